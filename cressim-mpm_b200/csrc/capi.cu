@@ -378,35 +378,7 @@ extern "C"
         }
         if (n > (unsigned)s->numMaxParticles)
             return bad("CrB200SolverCopyParticleState: n exceeds numMaxParticles");
-        if (int rc = s->residentSyncPlanes())
-            return rc;
-        const size_t stride = (size_t)s->numMaxParticles;
-        // planes -> per-particle 9 floats: a strided 2D copy per matrix
-        if (F)
-        {
-            for (int k = 0; k < 9; ++k)
-            {
-                cudaError_t e = cudaMemcpy2DAsync(F + k, 9 * sizeof(float), s->F + k * stride, sizeof(float), sizeof(float), n,
-                                      cudaMemcpyDeviceToDevice, s->stream);
-                if (e != cudaSuccess)
-                    return crb200::cudaFail(e, "copy F");
-            }
-        }
-        if (C)
-            for (int k = 0; k < 9; ++k)
-            {
-                cudaError_t e = cudaMemcpy2DAsync(C + k, 9 * sizeof(float), s->Cm + k * stride, sizeof(float),
-                                                  sizeof(float), n, cudaMemcpyDeviceToDevice, s->stream);
-                if (e != cudaSuccess)
-                    return crb200::cudaFail(e, "copy C");
-            }
-        if (V0)
-        {
-            cudaError_t e = cudaMemcpyAsync(V0, s->V0, n * sizeof(float), cudaMemcpyDeviceToDevice, s->stream);
-            if (e != cudaSuccess)
-                return crb200::cudaFail(e, "copy V0");
-        }
-        return CRB200_OK;
+        return s->copyParticleState(n, F, C, V0);
     }
 
     CRB200_API int CrB200SolverSetParticleState(CrB200SolverHandle solver, unsigned int n, const float *F,
@@ -420,33 +392,7 @@ extern "C"
         }
         if (n > (unsigned)s->numMaxParticles)
             return bad("CrB200SolverSetParticleState: n exceeds numMaxParticles");
-        if (int rc = s->residentRetire()) // the new state is read from the particle-id planes
-            return rc;
-        const size_t stride = (size_t)s->numMaxParticles;
-        for (int k = 0; k < 9; ++k)
-        {
-            if (F)
-            {
-                cudaError_t e = cudaMemcpy2DAsync(s->F + k * stride, sizeof(float), F + k, 9 * sizeof(float),
-                                                  sizeof(float), n, cudaMemcpyDeviceToDevice, s->stream);
-                if (e != cudaSuccess)
-                    return crb200::cudaFail(e, "set F");
-            }
-            if (C)
-            {
-                cudaError_t e = cudaMemcpy2DAsync(s->Cm + k * stride, sizeof(float), C + k, 9 * sizeof(float),
-                                                  sizeof(float), n, cudaMemcpyDeviceToDevice, s->stream);
-                if (e != cudaSuccess)
-                    return crb200::cudaFail(e, "set C");
-            }
-        }
-        if (V0)
-        {
-            cudaError_t e = cudaMemcpyAsync(s->V0, V0, n * sizeof(float), cudaMemcpyDeviceToDevice, s->stream);
-            if (e != cudaSuccess)
-                return crb200::cudaFail(e, "set V0");
-        }
-        return CRB200_OK;
+        return s->setParticleState(n, F, C, V0);
     }
 
     CRB200_API int CrB200SolverCopySortState(CrB200SolverHandle solver, unsigned int *keys, unsigned int *sortedIds,

@@ -312,6 +312,11 @@ namespace crb200
         int residentSyncPlanes();           // F, C back to the particle-id planes
         int residentRetire();               // planes synced, resident state dropped
         int copyCutMasks(unsigned *out);
+        // F, C, V0 of particles 0..n-1 (any of them null) to / from per-particle arrays
+        int copyParticleState(unsigned n, float *outF, float *outC, float *outV0);
+        int setParticleState(unsigned n, const float *inF, const float *inC, const float *inV0);
+        template <bool ToPlanes>
+        int moveMatrices(unsigned n, float *rowsF, float *rowsC);
     };
 
     // Grid of one scene (node counts as the reference's solver constructors compute them).

