@@ -40,13 +40,13 @@ class GeometrySdfDataC(C.Structure):
 
 def reference_root() -> str | None:
     """Where the reference's sources lie, as the oracle recipe (oracle/Makefile, `print-ref`) has
-    it; None when that folder does not exist (on a machine that only runs the prebuilt oracle)."""
+    it; None when that folder does not hold them (on a machine that only runs the prebuilt oracle)."""
     try:
         r = subprocess.run(["make", "-s", "-C", HERE, "print-ref"], capture_output=True, text=True, check=True)
     except (OSError, subprocess.CalledProcessError):
         return None
     path = r.stdout.strip()
-    return path if path and os.path.isdir(path) else None
+    return path if path and os.path.isdir(os.path.join(path, "src", "solver")) else None
 
 
 def build(ref: bool = True) -> None:
