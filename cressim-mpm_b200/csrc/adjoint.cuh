@@ -846,13 +846,9 @@ namespace crb200
 
     // State blob: x|m (float4 n), v (float4 n), F (9 planes of n), C (9 planes of n).
     // One kernel moves a particle state between the solver's arrays and a blob (x|m and v as
-    // float4, then F and C as 9 planes of n floats each); loading also clears the bin counters and
-    // the carried-records flag (what invalidateRecords does), so a replayed state costs one graph
-    // node instead of seven.
+    // float4, then F and C as 9 planes of n floats each).
     __global__ void k_stateCopy(unsigned n, unsigned stride, bool load, float4 *__restrict__ x, float4 *__restrict__ v,
-                                float *__restrict__ F, float *__restrict__ C, unsigned char *__restrict__ blob,
-                                unsigned *__restrict__ blockCount, unsigned numBlockCounts,
-                                unsigned *__restrict__ cellCount, unsigned numCellCounts, unsigned *__restrict__ flag)
+                                float *__restrict__ F, float *__restrict__ C, unsigned char *__restrict__ blob)
     {
         // the blob has the live arrays' layout (x, v, then the F and C planes, `stride` apart), so
         // the reverse kernels can read a saved state in place
@@ -886,18 +882,6 @@ namespace crb200
                     b[i] = a[i];
             }
         }
-        if (load)
-        {
-            for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < numBlockCounts; j += stepN)
-                blockCount[j] = 0u;
-            for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < numCellCounts; j += stepN)
-                cellCount[j] = 0u;
-            if (blockIdx.x == 0 && threadIdx.x == 0)
-            {
-                flag[0] = 0u; // recordsValid
-                flag[1] = 0u; // pbRecordsValid
-            }
-        }
     }
 
     int Solver::saveState(unsigned char *dst)
@@ -908,7 +892,7 @@ namespace crb200
         if (int r = residentSyncPlanes()) // F and C of the resident path into the particle-id planes
             return r;
         k_stateCopy<<<std::min((n + 255) / 256, 2u * (unsigned)strideCtas), 256, 0, stream>>>(
-            n, (unsigned)numMaxParticles, false, positionMass, velocity, F, Cm, dst, nullptr, 0u, nullptr, 0u, nullptr);
+            n, (unsigned)numMaxParticles, false, positionMass, velocity, F, Cm, dst);
         CRB_LAUNCHED(1);
         return CRB200_OK;
     }
@@ -921,10 +905,10 @@ namespace crb200
         resPlanesStale = false;
         CRB_CHECK(cudaMemsetAsync(&header->sortSkip, 0, sizeof(unsigned), stream));
         const unsigned n = totalParticles();
-        const unsigned nodes = totalBlocks * 64u;
-        k_stateCopy<<<std::max(1u, std::min((std::max(n, nodes) + 255) / 256, 2u * (unsigned)strideCtas)), 256, 0, stream>>>(
-            n, (unsigned)numMaxParticles, true, positionMass, velocity, F, Cm, const_cast<unsigned char *>(src),
-            blockCount, totalBlocks + 1, cellCount, nodes, &header->recordsValid);
+        if (!n)
+            return CRB200_OK;
+        k_stateCopy<<<std::min((n + 255) / 256, 2u * (unsigned)strideCtas), 256, 0, stream>>>(
+            n, (unsigned)numMaxParticles, true, positionMass, velocity, F, Cm, const_cast<unsigned char *>(src));
         CRB_LAUNCHED(1);
         return CRB200_OK;
     }
@@ -1073,7 +1057,7 @@ namespace crb200
         p += al((size_t)numMaxParticles * 4);
         t.cellStart = reinterpret_cast<unsigned *>(p);
         p += al(nodes * 4);
-        t.blockStart = reinterpret_cast<unsigned *>(p);
+        t.blockEnd = reinterpret_cast<unsigned *>(p);
         p += al(((size_t)totalBlocks + 1) * 4);
         t.activeList = reinterpret_cast<unsigned *>(p);
         p += al(((size_t)totalBlocks + 1) * 4);
@@ -1102,7 +1086,7 @@ namespace crb200
         CRB_CHECK(cudaMemsetAsync(gridG, 0, (size_t)totalBlocks * 64 * sizeof(float4), stream));
         k_adjG2P<Multi><<<pg, kAdjThreads, 0, stream>>>(p, sc, sx, activeMask, sF, stride, shapeTable, sp, ts.gridV, aX, aV, aF,
                                                 aC, gridG, records);
-        k_accumulate<0, Multi><<<p2gCtas, 64, 0, stream>>>(p, sc, ts.hdr, ts.activeList, ts.blockStart, ts.sortedIds,
+        k_accumulate<0, Multi><<<p2gCtas, 64, 0, stream>>>(p, sc, ts.hdr, ts.activeList, ts.blockEnd, ts.sortedIds,
                                                             ts.cellStart, records, cutMasks, gridG, gridF);
         k_adjGridUpdate<Multi><<<updCtas, 256, 0, stream>>>(p, sc, ts.hdr, ts.touchedList, shapeTable, sp, ts.gridA, gridG);
         k_adjP2G<Multi><<<pg, kAdjThreads, 0, stream>>>(p, sc, sx, sv, activeMask, matParams, sF, sC, V0, stride, gridG, aX, aV,
@@ -1246,7 +1230,10 @@ namespace crb200
             outC = next.C;
         }
         tapeActive = k;
-        const int r = last ? (isBatch() ? launchStepT<true>(true) : launchStepT<false>(true)) : launchStep();
+        // slot 0 follows a loaded state; the others a replay that carried its bins and records here
+        const bool carriedIn = k > 0;
+        const int r = !last ? launchStep(carriedIn, true)
+                            : (isBatch() ? launchStepT<true>(true, carriedIn, false) : launchStepT<false>(true, carriedIn, false));
         tapeActive = -1;
         outX = outV = nullptr;
         outF = outC = nullptr;
@@ -1310,6 +1297,9 @@ namespace crb200
         const bool graphs = stream != nullptr && !phaseTiming;
         if (graphs && (r = adjointGraphs(K)) != CRB200_OK)
             return r;
+        if ((r = cleanSort()) != CRB200_OK)
+            return r;
+        sortDirty = true; // until the last replay, which carries nothing
         for (int seg = (T - 1) / K; seg >= 0; --seg)
         {
             const int t0 = seg * K, t1 = std::min(T, t0 + K);
@@ -1352,6 +1342,7 @@ namespace crb200
                     return r;
             }
         }
+        sortDirty = false;
         return CRB200_OK;
     }
 } // namespace crb200

@@ -50,7 +50,9 @@ namespace crb200
     {
         const StepParams *params;            // numScenes entries
         const unsigned short *particleScene; // scene of each particle (0xFFFF: none)
+        const unsigned short *blockScene;    // scene of each grid block
         unsigned *flags;                     // SF_* shape flags per scene
+        unsigned *anyFlags;                  // those of all scenes together
         int numScenes;
         unsigned numParticles;               // particles covered by all scenes
     };
@@ -65,17 +67,16 @@ namespace crb200
         unsigned resMovers;
         unsigned touchedNodes;
         unsigned numSorted;
+        unsigned numListed; // blocks the binning listed for the next sort; 0 again after the grid update
         unsigned status;
         unsigned fp64Fallbacks;
         unsigned shapeFlags;
-        unsigned recordsValid;   // set by G2P when it binned the particles and wrote the next P2G records
-        unsigned pbRecordsValid; // PB-MPM: set by the G2P of an iteration that wrote the next iteration's records
         unsigned sortSkip;       // the sort kernels of this call return at once (resident path, no re-sort due)
         unsigned resForce;       // host: re-sort at the next resident call
         unsigned resFromPlanes;  // host: that re-sort takes F, C, V0 from the particle-id planes
         unsigned resOutside;     // particles of this call whose stencil left their block's window
         unsigned matMixed;       // the resident particles' materials differ (else matUniform holds them)
-        unsigned pad;
+        unsigned pad[2];
         float4 matUniform; // lambda, mu, type (int bits), 0
     };
 
@@ -131,6 +132,7 @@ namespace crb200
         std::vector<GridGeom> batchGeom;
         StepParams *dParams = nullptr;
         unsigned short *dParticleScene = nullptr;
+        unsigned short *dBlockScene = nullptr;
         unsigned *dSceneFlags = nullptr;
         bool isBatch() const { return !batch.empty(); }
         int numScenes() const { return isBatch() ? (int)batch.size() : 1; }
@@ -178,10 +180,14 @@ namespace crb200
         float4 *gridV = nullptr; // velocity grid
         float4 *gridF = nullptr; // node force (standard MPM)
         unsigned *keys = nullptr, *ranks = nullptr, *sortedIds = nullptr;
-        unsigned *cellCount = nullptr; // particles per cell (binning), cleared by k_cellStarts
+        // particles per cell and block (binning); zero outside a substep, the sort clears what it reads
+        unsigned *cellCount = nullptr;
         unsigned *cellStart = nullptr; // absolute first sorted slot of each cell of the active blocks
-        unsigned *blockCount = nullptr, *blockStart = nullptr;
+        unsigned *blockCount = nullptr;
+        unsigned *blockStart = nullptr; // block order of the slots (sortParticles): totalBlocks + 1
+        unsigned *blockEnd = nullptr;   // end of each active block's slots (substeps)
         unsigned *activeList = nullptr, *touchedList = nullptr;
+        unsigned *touchedFlag = nullptr; // per grid block: already in this substep's touched list
         unsigned *tileSums = nullptr;
         unsigned char *blockFlags = nullptr;
         unsigned long long *blockShapeMask = nullptr; // shapes that can reach each block's region (particles)
@@ -198,25 +204,25 @@ namespace crb200
         int strideCtas = 0;
         int cellCtas = 0;
 
-        cudaGraphExec_t graph = nullptr;
+        // One substep, by its place in a call: bit 0, the previous substep's G2P has binned the
+        // particles and written their P2G records; bit 1, this substep's G2P does so for the next
+        // one (MLS-MPM; the other solvers' substeps all bin and build for themselves).
+        cudaGraphExec_t graph[4] = {nullptr, nullptr, nullptr, nullptr};
         unsigned graphVersion = ~0u;
-        int graphKernels = 0;
-        // The substeps of a call but its last: their G2P leaves the velocity and C to the P2G record
-        // it writes for the next substep (leanG2P is set while this graph is captured).
-        cudaGraphExec_t graphLean = nullptr;
-        bool leanG2P = false;
-        // step(): the record invalidation and one substep
-        cudaGraphExec_t graphSingle = nullptr;
-        unsigned graphSingleVersion = ~0u;
-        int graphSingleKernels = 0;
+        int graphKernels[4] = {0, 0, 0, 0};
+        int substepGraph(int which);
+        // a call that set out to change the sort's counters has not ended well: clear them first
+        bool sortDirty = false;
+        int cleanSort();
+        int substeps(int n);
 
         StepParams params() const;
         SceneTable sceneTable() const;
         std::vector<StepParams> allParams() const;
         int uploadParams();
-        int launchStep();   // enqueue one step's kernels
+        int launchStep(bool carriedIn, bool carryOut); // enqueue one step's kernels
         template <bool Multi>
-        int launchStepT(bool recompute);
+        int launchStepT(bool recompute, bool carriedIn, bool carryOut);
 
         // adjoint of the MLS-MPM substep (CrB200SolverAdjointRecord / AdjointBackward)
         int adjointRecord(int numSubsteps, int interval, const int *captures, int numCaptures, float4 *capturedX);
@@ -230,7 +236,7 @@ namespace crb200
         struct TapeSlot
         {
             float4 *gridA, *gridV;
-            unsigned *sortedIds, *cellStart, *blockStart, *activeList, *touchedList;
+            unsigned *sortedIds, *cellStart, *blockEnd, *activeList, *touchedList;
             SortHeader *hdr;
         };
         unsigned char *adjTape = nullptr;
@@ -250,7 +256,6 @@ namespace crb200
         void releaseAdjoint();
         int adjointCheck();
         int saveState(unsigned char *dst);
-        int invalidateRecords();
         int loadState(const unsigned char *src);
 
         // one saved state (x, v, F, C) in the layout of the live arrays
@@ -266,7 +271,7 @@ namespace crb200
         float *aF = nullptr, *aC = nullptr;                   // adjoint of F, C (planes of stride numMaxParticles)
         float4 *gridG = nullptr;                               // adjoint of the grid velocity / momentum and mass
         float4 *adjForce = nullptr, *adjTorque = nullptr;      // coupling output of recomputed substeps
-        int sortParticles(const StepParams &p, bool ignoreMask);
+        int sortParticles(const StepParams &p, bool ignoreMask, bool honourSkip);
         void gatherShapes(cudaStream_t s);
         bool detCoupling = false;            // CRB200_OPT_DETERMINISTIC_COUPLING
         float4 *detPartials = nullptr;       // per block and dynamic slot: force, torque partial sums
@@ -277,8 +282,6 @@ namespace crb200
         int setDeterministicCoupling(bool on);
         int setDeterministic(bool on);
         int detLevel(bool recomputing) const;
-        cudaStream_t sideStream = nullptr; // shape gather / cut masks beside the sort chain
-        cudaEvent_t forkEvent = nullptr, joinEvent = nullptr;
 
         // Resident path (single-scene MLS-MPM): particle state kept in cell order between substeps,
         // one fused kernel per substep for G2P of substep k and P2G of substep k + 1, a re-sort only
@@ -295,7 +298,6 @@ namespace crb200
         float4 *resX2 = nullptr, *resMat2 = nullptr; // re-sort scratch
         float *resV02 = nullptr, *resF2 = nullptr, *resC2 = nullptr;
         unsigned *resId2 = nullptr, *resSlotOf = nullptr;
-        unsigned *touchedFlag = nullptr;    // per grid block: already in this substep's touched list
         int resCtas = 0;                    // CTAs of the fused kernel: occupancy x SMs x resMult
         int resMult = 1;                    // autotuned
         cudaGraphExec_t resGraph[3] = {nullptr, nullptr, nullptr}; // call start, middle substep, last substep

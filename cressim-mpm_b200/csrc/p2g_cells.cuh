@@ -264,33 +264,80 @@ namespace crb200
         }
     }
 
-    // (b) One record per particle (indexed by particle id), particle-parallel over the sorted slots.
-    //     Outliers are scattered here with global atomics and leave a zero record.  PB-MPM's
-    //     material constraint writes the relaxed C back.  Nothing to do when the previous substep's
-    //     G2P already wrote the records (hdr->recordsValid; PB-MPM: hdr->pbRecordsValid).
+    // (b) Every binned particle into its cell's slots, and its P2G record (indexed by particle id)
+    //     unless the previous substep's G2P wrote it (carried; a scene with a slicer carries none,
+    //     since its records follow the cut masks, which are evaluated here for MLS-MPM).  Outliers
+    //     are scattered with global atomics and leave a zero record.  PB-MPM's material constraint
+    //     writes the relaxed C back.
+    //     Placing alone is a chain of three dependent accesses per particle: where nothing but that
+    //     is left to do (carried, no slicer in any scene), a thread takes kPlacePer particles, so
+    //     that as many chains are in flight, and the CTAs past the last particle exit.  @PLACE@
+    constexpr unsigned kPlacePer = 4, kPlaceThreads = 256;
     template <int Mode, bool Multi>
-    __global__ void __launch_bounds__(128, Mode == 1 ? 4 : 8) k_record(const __grid_constant__ StepParams p0, SceneTable sc,
-                                                    const SortHeader *__restrict__ hdr,
-                                                    const unsigned *__restrict__ sortedIds, const float4 *__restrict__ xm,
+    __global__ void __launch_bounds__(kPlaceThreads, Mode == 1 ? 2 : 4) k_place(const __grid_constant__ StepParams p0, SceneTable sc,
+                                                    bool carried, const unsigned *__restrict__ keys,
+                                                    const unsigned *__restrict__ ranks, const unsigned *__restrict__ cellStart,
+                                                    unsigned *__restrict__ sortedIds, unsigned capacity,
+                                                    const float4 *__restrict__ xm,
                                                     const float4 *__restrict__ vel, const float4 *__restrict__ matParams,
                                                     const int *__restrict__ matType, const float *__restrict__ F,
                                                     float *__restrict__ Cm, const float *__restrict__ V0, unsigned stride,
-                                                    const unsigned *__restrict__ cutMasks, float4 *__restrict__ records,
+                                                    const ShapeRec *__restrict__ shapeTable, SdfPtrs sdf,
+                                                    unsigned *__restrict__ cutMasks, float4 *__restrict__ records,
                                                     float4 *__restrict__ gridA, float4 *__restrict__ gridF, unsigned *fp64Count)
     {
-        if ((Mode == 0 && !Multi && hdr->recordsValid) || (Mode == 1 && hdr->pbRecordsValid))
+        const unsigned n = Multi ? sc.numParticles : p0.numActive;
+        const bool anyCut = Mode == 0 && (Multi || p0.numShapes > 0) && (*sc.anyFlags & SF_SLICER);
+        const bool cutScene = !Multi && anyCut;
+        const bool placeOnly = Mode == 0 && carried && !anyCut;
+        const unsigned per = placeOnly ? kPlacePer : 1u;
+        const unsigned i0 = blockIdx.x * kPlaceThreads * per + threadIdx.x;
+        if (blockIdx.x * kPlaceThreads * per >= n)
             return;
-        const bool carry = Mode == 0 && Multi && hdr->recordsValid;
-        const unsigned nS = hdr->numSorted;
-        for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < nS; j += gridDim.x * blockDim.x)
+        unsigned key[kPlacePer], slot[kPlacePer];
+#pragma unroll
+        for (unsigned e = 0; e < kPlacePer; ++e)
         {
-        const unsigned id = sortedIds[j];
+            const unsigned i = i0 + kPlaceThreads * e;
+            key[e] = e < per && i < n ? keys[i] : kInvalidKey;
+            slot[e] = key[e] != kInvalidKey ? ranks[i] : 0u;
+        }
+#pragma unroll
+        for (unsigned e = 0; e < kPlacePer; ++e)
+            if (key[e] != kInvalidKey)
+                slot[e] += cellStart[key[e]];
+#pragma unroll
+        for (unsigned e = 0; e < kPlacePer; ++e)
+            if (key[e] != kInvalidKey && slot[e] < capacity) // always, unless the counts were inconsistent (flagged)
+                sortedIds[slot[e]] = i0 + kPlaceThreads * e;
+        if (placeOnly)
+            return;
+        __shared__ ShapeRec sh[Mode == 0 && !Multi ? kMaxShapes : 1];
+        if (cutScene)
+        {
+            loadShapes(sh, shapeTable, p0.numShapes);
+            __syncthreads();
+        }
+        const unsigned id = i0;
+        if (key[0] == kInvalidKey)
+            return;
         const unsigned si = Multi ? sc.particleScene[id] : 0u; // sorted particles have a scene
-        if (carry && !(sc.flags[si] & SF_SLICER))
-            continue; // the previous G2P wrote this particle's record
         const StepParams &p = Multi ? sc.params[si] : p0;
         const bool slicers = Mode <= 1 && p.numShapes > 0 && (sc.flags[si] & SF_SLICER);
-        const unsigned msk = slicers ? cutMasks[id] : 0u;
+        if (Mode == 0 && carried && !slicers)
+            return; // the previous G2P wrote this particle's record
+        unsigned msk = 0u;
+        if (slicers)
+        {
+            if (Mode == 0)
+            {
+                const V3 x = v3(xm[id]);
+                msk = cutMaskOf(p.g, x, stencilOf(p.g, x), Multi ? shapeTable + p.shapeBegin : sh, p.numShapes, sdf);
+                cutMasks[id] = msk;
+            }
+            else
+                msk = cutMasks[id];
+        }
         RawParticle raw;
         loadRaw<Mode>(id, xm, vel, matParams, matType, F, Cm, V0, stride, raw);
         float rec[kRec];
@@ -305,7 +352,6 @@ namespace crb200
         out[1] = make_float4(rec[4], rec[5], rec[6], rec[7]);
         out[2] = make_float4(rec[8], rec[9], rec[10], rec[11]);
         out[3] = make_float4(rec[12], rec[13], rec[14], rec[15]);
-        }
     }
 
     __device__ __forceinline__ void loadRecord(const float4 *__restrict__ records, unsigned j, float rec[kRec])
@@ -319,7 +365,7 @@ namespace crb200
     }
 
     // (c) Cell accumulation: one 64-thread CTA per active block, one thread per cell.
-    //     Multi: each active block reads its scene's parameters (block base search).
+    //     Multi: each active block reads its scene's parameters.
     //     Det: nothing is added atomically.  A cell thread accumulates all of its cell's particles
     //     (no kCellRun cap) and the block's whole 6x6x6 tile is stored to tiles[block] (tilesF for
     //     the standard solver's force pass), from which the grid update sums each node's sources in
@@ -327,7 +373,7 @@ namespace crb200
     template <int Mode, bool Multi, bool Det = false>
     __global__ void __launch_bounds__(64, Multi ? 5 : 6) k_accumulate(const __grid_constant__ StepParams p0, SceneTable sc, const SortHeader *__restrict__ hdr,
                                                        const unsigned *__restrict__ activeList,
-                                                       const unsigned *__restrict__ blockStart,
+                                                       const unsigned *__restrict__ blockEnd,
                                                        const unsigned *__restrict__ sortedIds,
                                                        const unsigned *__restrict__ cellStart,
                                                        const float4 *__restrict__ records,
@@ -365,7 +411,7 @@ namespace crb200
             const bool slicers = Mode <= 1 && p.numShapes > 0 && (sc.flags[si] & SF_SLICER);
             const unsigned lb = b - g.blockBase;
             const int bx = lb % g.nb.x, by = (lb / g.nb.x) % g.nb.y, bz = lb / (g.nb.x * g.nb.y);
-            const unsigned start = blockStart[b], cnt = blockStart[b + 1] - start;
+            const unsigned start = cellStart[b * 64u], cnt = blockEnd[b] - start;
             // cell ranges of this block's sorted slots (cells are contiguous, in cell order)
             {
                 const unsigned excl = cellStart[b * 64u + tid] - start;

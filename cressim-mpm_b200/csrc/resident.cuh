@@ -47,12 +47,6 @@ namespace crb200
     };
     static_assert(sizeof(ResShared) % 16 == 0, "shapes follow ResShared in shared memory");
 
-    __device__ __forceinline__ void markTouched(unsigned blk, unsigned *__restrict__ touchedFlag,
-                                                unsigned *__restrict__ touchedList, SortHeader *hdr)
-    {
-        if (atomicExch(&touchedFlag[blk], 1u) == 0u)
-            touchedList[atomicAdd(&hdr->numTouchedBlocks, 1u)] = blk;
-    }
 
     // A record passed by value, so that the caller's copy stays in registers.
     struct RecVal

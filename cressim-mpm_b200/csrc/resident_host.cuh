@@ -46,10 +46,8 @@ namespace crb200
         CRB_CHECK(cudaMalloc(&resF2, 9 * n * sizeof(float)));
         CRB_CHECK(cudaMalloc(&resC2, 9 * n * sizeof(float)));
         CRB_CHECK(cudaMalloc(&resId2, n * sizeof(unsigned)));
-        CRB_CHECK(cudaMalloc(&touchedFlag, (size_t)totalBlocks * sizeof(unsigned)));
         CRB_CHECK(cudaMemsetAsync(res.cut, 0, n * sizeof(unsigned), stream));
         CRB_CHECK(cudaMemsetAsync(resSlotOf, 0xff, n * sizeof(unsigned), stream));
-        CRB_CHECK(cudaMemsetAsync(touchedFlag, 0, (size_t)totalBlocks * sizeof(unsigned), stream));
         const int maxSmem = (int)(sizeof(ResShared) + kMaxShapes * sizeof(ShapeRec));
         CRB_CHECK(cudaFuncSetAttribute(k_g2p2g<false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxSmem));
         CRB_CHECK(cudaFuncSetAttribute(k_g2p2g<true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxSmem));
@@ -144,7 +142,7 @@ namespace crb200
             }
             k_resDecide<<<1, 1, 0, stream>>>(header);
             CRB_LAUNCHED(1);
-            if ((r = sortParticles(p, false)) != CRB200_OK)
+            if ((r = sortParticles(p, false, true)) != CRB200_OK)
                 return r;
             k_resGather<<<strideCtas, 256, 0, stream>>>(header, sortedIds, positionMass, velocity, matParams, matType, F,
                                                          Cm, V0, res, resSlotOf, resX2, resV02, resF2, resC2, resMat2,
@@ -220,9 +218,10 @@ namespace crb200
             CRB_CHECK(cudaMemsetAsync(&header->resForce, 1, 2 * sizeof(unsigned), stream));
             resValid = true;
         }
-        int r = invalidateRecords();
+        int r = cleanSort();
         if (r != CRB200_OK)
             return r;
+        sortDirty = false; // a resident call sorts once, in block order, and leaves the counters zero
         if (stream == nullptr || phaseTiming)
         {
             if (phaseTiming)
