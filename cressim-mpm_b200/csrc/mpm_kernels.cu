@@ -1147,7 +1147,7 @@ namespace crb200
     //    state); particles whose new stencil leaves the grid are scattered into the (cleared)
     //    accumulation grid here, as k_place does.  PB-MPM: the next iteration's record.
     template <int Mode, bool Multi>
-    __global__ void __launch_bounds__(128, Mode == 1 ? 4 : ((Mode == 0 && !Multi) ? 7 : 6)) k_g2p(const __grid_constant__ StepParams p0, SceneTable sc, float4 *xm,
+    __global__ void __launch_bounds__(128, Mode == 1 ? 5 : ((Mode == 0 && !Multi) ? 7 : 6)) k_g2p(const __grid_constant__ StepParams p0, SceneTable sc, float4 *xm,
                                                  float4 *vel, const unsigned char *__restrict__ mask,
                                                  float *F, float *Cm, unsigned stride,
                                                  const ShapeRec *__restrict__ shapeTable, SdfPtrs sdf,
@@ -1332,12 +1332,16 @@ namespace crb200
         const V3 va = S;
         if (Mode == 1)
         {
-            vel[i] = make_float4(va.x, va.y, va.z, 0.f);
-            storeM3(Cm, stride, i, Cn);
-            if (records)
+            // Between iterations v and C live in the record; v is read again only where the next G2P
+            // reflects it at a cut node.  The last iteration writes both.
+            if (!records || msk)
+                vel[i] = make_float4(va.x, va.y, va.z, 0.f);
+            if (!records)
+                storeM3(Cm, stride, i, Cn);
+            else
             {
-                // the next iteration's P2G record: the material constraint on the new C (which
-                // stores the relaxed C) and the record, as k_record would build them
+                // the next iteration's P2G record: the material constraint on the new C and the
+                // record, as k_place would build them
                 RawParticle raw;
                 raw.x4 = x4;
                 raw.v4 = make_float4(va.x, va.y, va.z, 0.f);
@@ -1353,17 +1357,19 @@ namespace crb200
                 }
                 raw.v0 = 0.f;
                 float rec[kRec];
-                if (!buildRecord<1>(p, i, raw, Cm, stride, msk, true, gridA, nullptr, &hdr->fp64Fallbacks, rec))
+                const int built = buildRecord<1, false>(p, i, raw, msk, true, gridA, nullptr, nullptr, rec);
+                if (built < 0)
+                {
+                    pbRecordSvd(p, i, raw, msk, gridA, &hdr->fp64Fallbacks, records);
+                    return;
+                }
+                if (!built)
                 {
 #pragma unroll
                     for (int e = 0; e < kRec; ++e)
                         rec[e] = 0.f;
                 }
-                float4 *out = records + 4ull * i;
-                out[0] = make_float4(rec[0], rec[1], rec[2], rec[3]);
-                out[1] = make_float4(rec[4], rec[5], rec[6], rec[7]);
-                out[2] = make_float4(rec[8], rec[9], rec[10], rec[11]);
-                out[3] = make_float4(rec[12], rec[13], rec[14], rec[15]);
+                storeRecord(records + 4ull * i, rec);
             }
             return;
         }
@@ -1410,7 +1416,7 @@ namespace crb200
             }
             raw.v0 = V0[i];
             float rec[kRec];
-            if (!buildRecord<0>(p, i, raw, nullptr, stride, 0u, true, gridA, nullptr, nullptr, rec))
+            if (!buildRecord<0>(p, i, raw, 0u, true, gridA, nullptr, nullptr, rec))
             {
 #pragma unroll
                 for (int e = 0; e < kRec; ++e)
@@ -2220,20 +2226,35 @@ namespace crb200
         const unsigned pg = (nPart + 127) / 128;
         const bool det2 = detLevel(recompute || adjReplay) == 2;
         int r = CRB200_OK;
-        if (!carriedIn)
+        const bool solves = !(isPb && iterations <= 0);
+        if (!solves)
         {
-            k_bin<Multi><<<std::max(pg, 1u), 128, 0, stream>>>(p, sc, isStd, false, positionMass, activeMask, keys, ranks,
-                                                               blockCount, cellCount, activeList, header);
+            // PB-MPM without iterations only integrates the particles.  The grid update, which takes the
+            // block lists back, does not run, so the sort is the block-ordered one.
+            if (numShapes > 0)
+            {
+                gatherShapes(stream);
+                CRB_LAUNCHED(1);
+            }
+            if ((r = sortParticles(p, false, false)) != CRB200_OK)
+                return r;
+        }
+        else
+        {
+            if (!carriedIn)
+            {
+                k_bin<Multi><<<std::max(pg, 1u), 128, 0, stream>>>(p, sc, isStd, false, positionMass, activeMask, keys,
+                                                                   ranks, blockCount, cellCount, activeList, header);
+                CRB_LAUNCHED(1);
+            }
+            if (det2)
+                CRB_CHECK(cudaMemsetAsync(blockFlags, 0, totalBlocks, stream));
+            const int shapeCtas = numShapes > 0 ? numScenes() : 0;
+            k_sortBlocks<<<shapeCtas + cellCtas, 256, 0, stream>>>(
+                p, sc, shapeCtas, shapeIds, shapes, geometries, shapeTable, activeList, blockCount, cellCount, cellStart,
+                blockEnd, det2 ? blockFlags : nullptr, touchedFlag, touchedList, (unsigned)numMaxParticles, header);
             CRB_LAUNCHED(1);
         }
-        if (det2)
-            CRB_CHECK(cudaMemsetAsync(blockFlags, 0, totalBlocks, stream));
-        const int shapeCtas = numShapes > 0 ? numScenes() : 0;
-        k_sortBlocks<<<shapeCtas + cellCtas, 256, 0, stream>>>(p, sc, shapeCtas, shapeIds, shapes, geometries, shapeTable,
-                                                              activeList, blockCount, cellCount, cellStart, blockEnd,
-                                                              det2 ? blockFlags : nullptr, touchedFlag, touchedList,
-                                                              (unsigned)numMaxParticles, header);
-        CRB_LAUNCHED(1);
         // Slicer cut masks of this step's positions (positions do not change across PB-MPM
         // iterations, so one evaluation serves every iteration; MLS-MPM's k_place evaluates them).
         if (numShapes > 0 && isPb && pg)
@@ -2257,13 +2278,13 @@ namespace crb200
         };
         if (isStd)
             r = place(std::integral_constant<int, 2>{});
-        else if (isPb)
-            r = place(std::integral_constant<int, 1>{});
-        else
+        else if (!isPb)
             r = place(std::integral_constant<int, 0>{});
+        else if (solves)
+            r = place(std::integral_constant<int, 1>{});
         if (r != CRB200_OK)
             return r;
-        if (nPart > 0 && det2)
+        if (nPart > 0 && det2 && solves)
         {
             k_cellOrder<<<cellCtas * 4, 64, 0, stream>>>(header, activeList, blockEnd, cellStart, sortedIds);
             CRB_LAUNCHED(1);

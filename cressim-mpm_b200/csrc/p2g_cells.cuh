@@ -99,13 +99,13 @@ namespace crb200
     // Record of one particle for the cell accumulation:
     //   [0..2] u, [3] m, [4..12] a0 a1 a2 (MLS / PB) or -V0*tau column-major (standard force),
     //   [13..15] fx.
-    // Returns false when the particle must not go through the cell path (non-finite position or a
+    // Returns 0 when the particle must not go through the cell path (non-finite position or a
     // stencil base outside [0, n-2]); such particles are scattered here with global atomics when
-    // scatterOutliers is set.
-    template <int Mode>
-    __device__ __forceinline__ bool buildRecord(const StepParams &p, unsigned id, const RawParticle &raw,
-                                                float *__restrict__ Cm, unsigned stride, unsigned cutMask,
-                                                bool scatterOutliers, float4 *__restrict__ gridA,
+    // scatterOutliers is set.  PB-MPM without Svd: -1, and nothing done, when the particle's rotation
+    // needs the SVD.
+    template <int Mode, bool Svd = true>
+    __device__ __forceinline__ int buildRecord(const StepParams &p, unsigned id, const RawParticle &raw,
+                                                unsigned cutMask, bool scatterOutliers, float4 *__restrict__ gridA,
                                                 float4 *__restrict__ gridF, unsigned *fp64Count, float rec[kRec])
     {
         const GridGeom &g = p.g;
@@ -115,7 +115,7 @@ namespace crb200
         for (int e = 0; e < kRec; ++e)
             rec[e] = 0.f;
         if (!st.finite)
-            return false;
+            return 0;
         const V3 v = v3(raw.v4);
         M3 Fp;
 #pragma unroll
@@ -148,7 +148,11 @@ namespace crb200
                     for (int e = 0; e < 9; ++e)
                         tF.m[e] = Cp.m[e] * p.dt + ((e % 4) == 0 ? 1.f : 0.f);
                     tF = matmul(tF, Fp);
-                    const M3 R = pbRotationTarget(tF, fp64Count);
+                    M3 R;
+                    if (Svd)
+                        R = pbRotationTarget(tF, fp64Count);
+                    else if (!pbRotationNear(tF, R))
+                        return -1;
                     const float detF = det3(tF);
                     const float cd = fminf(fmaxf(fabsf(detF), 0.1f), 1000.0f);
                     const float qs = 1.0f / (copysignf(1.0f, detF) * sqrtf(cd));
@@ -160,7 +164,6 @@ namespace crb200
 #pragma unroll
                     for (int e = 0; e < 9; ++e)
                         Cp.m[e] = Cp.m[e] + ((TF.m[e] - ((e % 4) == 0 ? 1.f : 0.f)) - Cp.m[e] * p.dt) * raw.mp.x;
-                    storeM3(Cm, stride, id, Cp);
                 }
 #pragma unroll
                 for (int e = 0; e < 9; ++e)
@@ -197,7 +200,7 @@ namespace crb200
         if (!inside)
         {
             if (!scatterOutliers)
-                return false;
+                return 0;
             if (Mode == 2)
             {
                 scatterGlobal<2>(p, st, rec, 0u, gridA, gridF);
@@ -205,9 +208,33 @@ namespace crb200
             }
             else
                 scatterGlobal<Mode>(p, st, rec, cutMask, gridA, gridF);
-            return false;
+            return 0;
         }
-        return true;
+        return 1;
+    }
+
+    __device__ __forceinline__ void storeRecord(float4 *__restrict__ out, const float rec[kRec])
+    {
+        out[0] = make_float4(rec[0], rec[1], rec[2], rec[3]);
+        out[1] = make_float4(rec[4], rec[5], rec[6], rec[7]);
+        out[2] = make_float4(rec[8], rec[9], rec[10], rec[11]);
+        out[3] = make_float4(rec[12], rec[13], rec[14], rec[15]);
+    }
+
+    // PB-MPM record of a particle whose rotation needs the SVD: out of line, so that its registers
+    // do not limit the kernel around it.
+    static __device__ __noinline__ void pbRecordSvd(const StepParams &p, unsigned id, RawParticle raw, unsigned msk,
+                                                    float4 *__restrict__ gridA, unsigned *fp64Count,
+                                                    float4 *__restrict__ records)
+    {
+        float rec[kRec];
+        if (!buildRecord<1>(p, id, raw, msk, true, gridA, nullptr, fp64Count, rec))
+        {
+#pragma unroll
+            for (int e = 0; e < kRec; ++e)
+                rec[e] = 0.f;
+        }
+        storeRecord(records + 4ull * id, rec);
     }
 
     // Adds one particle's 27 node contributions to the cell thread's registers.
@@ -267,8 +294,8 @@ namespace crb200
     // (b) Every binned particle into its cell's slots, and its P2G record (indexed by particle id)
     //     unless the previous substep's G2P wrote it (carried; a scene with a slicer carries none,
     //     since its records follow the cut masks, which are evaluated here for MLS-MPM).  Outliers
-    //     are scattered with global atomics and leave a zero record.  PB-MPM's material constraint
-    //     writes the relaxed C back.
+    //     are scattered with global atomics and leave a zero record.  PB-MPM's relaxed C lives in the
+    //     record only: G2P replaces C in the same iteration.
     //     Placing alone is a chain of three dependent accesses per particle: where nothing but that
     //     is left to do (carried, no slicer in any scene), a thread takes kPlacePer particles, so
     //     that as many chains are in flight, and the CTAs past the last particle exit.  @PLACE@
@@ -281,7 +308,7 @@ namespace crb200
                                                     const float4 *__restrict__ xm,
                                                     const float4 *__restrict__ vel, const float4 *__restrict__ matParams,
                                                     const int *__restrict__ matType, const float *__restrict__ F,
-                                                    float *__restrict__ Cm, const float *__restrict__ V0, unsigned stride,
+                                                    const float *__restrict__ Cm, const float *__restrict__ V0, unsigned stride,
                                                     const ShapeRec *__restrict__ shapeTable, SdfPtrs sdf,
                                                     unsigned *__restrict__ cutMasks, float4 *__restrict__ records,
                                                     float4 *__restrict__ gridA, float4 *__restrict__ gridF, unsigned *fp64Count)
@@ -341,7 +368,7 @@ namespace crb200
         RawParticle raw;
         loadRaw<Mode>(id, xm, vel, matParams, matType, F, Cm, V0, stride, raw);
         float rec[kRec];
-        if (!buildRecord<Mode>(p, id, raw, Cm, stride, msk, true, gridA, gridF, fp64Count, rec))
+        if (!buildRecord<Mode>(p, id, raw, msk, true, gridA, gridF, fp64Count, rec))
         {
 #pragma unroll
             for (int e = 0; e < kRec; ++e)

@@ -343,7 +343,7 @@ namespace crb200
                     }
                     float rec[kRec];
                     // false: non-finite, or a base cell outside [0, n-2] (then nothing was scattered)
-                    const bool inside = buildRecord<0>(p, id, raw, nullptr, rs.stride, msk, false, nullptr, nullptr,
+                    const bool inside = buildRecord<0>(p, id, raw, msk, false, nullptr, nullptr,
                                                        nullptr, rec);
                     // The particle's current cell, when it lies in this block: the cell's threads sum
                     // its record, at a rank taken from the cell's shared counter (one atomic per group
