@@ -823,8 +823,13 @@ namespace crb200
     //    Det == 2: the P2G grid comes from the cell blocks' tiles (k_accumulate<.., true>): each
     //    node sums the tiles that cover it in a fixed order (gatherTiles), then what per-particle
     //    atomics left in gridA (particles whose stencil leaves the grid).
+    //    Bound by latency (block id, then its node sums, then contact), at 3 CTAs per SM: each block's
+    //    id and sums are read while its predecessor is worked on, the shapes are staged behind the
+    //    first of these reads, and the touched nodes are counted in registers.  30 -> 17 us a substep on
+    //    the 1.6M-particle slab, 56 -> 25 us over 64 scenes, 18 -> 13 us a PB-MPM iteration at 540k
+    //    particles; 4 CTAs per SM (64 registers, spills) gain nothing on that.
     template <bool Multi, int Det>
-    __global__ void __launch_bounds__(256) k_gridUpdate(const __grid_constant__ StepParams p0, SceneTable sc, const SortHeader *__restrict__ hdr,
+    __global__ void __launch_bounds__(256, 3) k_gridUpdate(const __grid_constant__ StepParams p0, SceneTable sc, const SortHeader *__restrict__ hdr,
                                                         const unsigned *__restrict__ touchedList,
                                                         const ShapeRec *__restrict__ shapeTable, SdfPtrs sdf,
                                                         float4 *__restrict__ gridA, float4 *__restrict__ gridF,
@@ -847,14 +852,27 @@ namespace crb200
         __shared__ float sCouple[kRows ? 256 : 1][kDetSlots * 6];
         if (threadIdx.x == 0)
             sTouched = 0;
-        if (!Multi && p0.numShapes > 0)
-            loadShapes(sh, shapeTable, p0.numShapes);
         if (blockIdx.x == 0 && threadIdx.x == 0)
             const_cast<SortHeader *>(hdr)->numListed = 0u; // the sort has read it; G2P lists anew
-        __syncthreads();
         const unsigned nT = hdr->numTouchedBlocks;
         const bool withForce = p0.solverType == CRB200_SOLVER_GPU_STANDARD;
         const unsigned perCta = blockDim.x / 64;
+        unsigned touched = 0; // this thread's nodes that received mass
+        // the first block's id and sums; each later one is read while its predecessor is worked on
+        unsigned nextB = 0;
+        float4 nextAcc = make_float4(0.f, 0.f, 0.f, 0.f);
+        auto fetch = [&](unsigned bi) {
+            if (bi < nT)
+            {
+                nextB = touchedList[bi];
+                nextAcc = gridA[nextB * 64u + (threadIdx.x & 63)];
+            }
+        };
+        fetch(blockIdx.x * perCta + threadIdx.x / 64);
+        // the shapes arrive while those reads are under way
+        if (!Multi && p0.numShapes > 0 && blockIdx.x * perCta < nT)
+            loadShapes(sh, shapeTable, p0.numShapes);
+        __syncthreads();
         using Couple = typename std::conditional<kRows, CoupleRow, CoupleAtomic>::type;
         if constexpr (kRows)
             for (int c = 0; c < kDetSlots * 6; ++c)
@@ -867,13 +885,14 @@ namespace crb200
                 couple = CoupleRow{sCouple[threadIdx.x], CoupleAtomic{coupleForce, coupleTorque}, false};
             else
                 couple = CoupleAtomic{coupleForce, coupleTorque};
-            unsigned b = 0;
+            const unsigned b = nextB;
+            float4 acc = nextAcc;
+            fetch(bi + gridDim.x * perCta);
             // one node of block touchedList[bi]; leaves early where the reference's update returns
             do
             {
                 if (bi >= nT)
                     break;
-                b = touchedList[bi];
                 if ((threadIdx.x & 63) == 0)
                     touchedFlag[b] = 0u;
                 const StepParams &p = Multi ? sc.params[sceneOfBlock(sc, b)] : p0;
@@ -900,7 +919,6 @@ namespace crb200
                 if (!inGrid(g, i, j, k))
                     break;
                 const unsigned a = b * 64u + l;
-                float4 acc = gridA[a];
                 if (clearA)
                     gridA[a] = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (Det == 2)
@@ -915,13 +933,8 @@ namespace crb200
                     if (Det == 2)
                         f = gatherTiles(g, tilesF, blockFlags, bx, by, bz, l, f);
                 }
-                {
-                    // nodes that received mass (roofline bookkeeping): a shared counter per CTA
-                    const unsigned am = __activemask();
-                    const unsigned hit = __ballot_sync(am, acc.w > 0.f);
-                    if ((threadIdx.x & 31) == (unsigned)(__ffs(am) - 1) && hit)
-                        atomicAdd(&sTouched, (unsigned)__popc(hit));
-                }
+                if (acc.w > 0.f)
+                    ++touched; // nodes that received mass (roofline bookkeeping)
                 if (acc.w < p.cutoff)
                 {
                     gridV[a] = acc; // light nodes keep momentum, which G2P then reads (reference Q2)
@@ -979,6 +992,9 @@ namespace crb200
                 }
             }
         }
+        touched = __reduce_add_sync(0xffffffffu, touched);
+        if ((threadIdx.x & 31) == 0 && touched)
+            atomicAdd(&sTouched, touched);
         __syncthreads();
         if (threadIdx.x == 0 && sTouched)
             atomicAdd(&const_cast<SortHeader *>(hdr)->touchedNodes, sTouched);
@@ -2269,7 +2285,8 @@ namespace crb200
                 return CRB200_OK;
             // (a scene without shapes has no slicer: no CTA more than placing needs)
             const unsigned per = M == 0 && !Multi && carriedIn && numShapes == 0 ? kPlacePer : 1u;
-            k_place<M, Multi><<<(nPart + kPlaceThreads * per - 1) / (kPlaceThreads * per), kPlaceThreads, 0, stream>>>(
+            const unsigned placeCtas = (nPart + kPlaceThreads * per - 1) / (kPlaceThreads * per);
+            k_place<M, Multi><<<placeCtas, kPlaceThreads, 0, stream>>>(
                 p, sc, carriedIn, keys, ranks, cellStart, sortedIds, (unsigned)numMaxParticles, positionMass, velocity,
                 matParams, matType, F, Cm, V0, stride, shapeTable, sp, cutMasks, records, gridA, gridF,
                 &header->fp64Fallbacks);
