@@ -159,6 +159,7 @@ namespace crb200
                                                    const float *__restrict__ aC, float4 *__restrict__ gridG,
                                                    float4 *__restrict__ records)
     {
+        chainStart(p0.earlyNext);
         __shared__ ShapeRec sh[Multi ? 1 : kMaxShapes];
         // the particle's streams, staged at entry (launched with kAdjThreads threads)
         __shared__ float4 sX[kAdjThreads], sAx[kAdjThreads], sAv[kAdjThreads];
@@ -513,6 +514,7 @@ namespace crb200
                                                           const ShapeRec *__restrict__ shapeTable, SdfPtrs sdf,
                                                           float4 *__restrict__ gridA, float4 *__restrict__ gridG)
     {
+        chainStart(p0.earlyNext);
         __shared__ ShapeRec sh[Multi ? 1 : kMaxShapes];
         if (!Multi && p0.numShapes > 0)
             loadShapes(sh, shapeTable, p0.numShapes);
@@ -665,6 +667,7 @@ namespace crb200
                                                    float *__restrict__ aF, float *__restrict__ aC,
                                                    float4 *__restrict__ aMat)
     {
+        chainStart(p0.earlyNext);
         // the particle's streams, staged at entry (launched with kAdjThreads threads)
         __shared__ float4 sX[kAdjThreads], sVel[kAdjThreads], sMp[kAdjThreads], sAx[kAdjThreads], sAm[kAdjThreads];
         __shared__ float sF[9][kAdjThreads], sC[9][kAdjThreads], sAF[9][kAdjThreads], sV0[kAdjThreads];
@@ -1084,12 +1087,12 @@ namespace crb200
                          reinterpret_cast<const float4 *>(sdf.gradientSignedDistance)};
         const unsigned stride = (unsigned)numMaxParticles;
         CRB_CHECK(cudaMemsetAsync(gridG, 0, (size_t)totalBlocks * 64 * sizeof(float4), stream));
-        k_adjG2P<Multi><<<pg, kAdjThreads, 0, stream>>>(p, sc, sx, activeMask, sF, stride, shapeTable, sp, ts.gridV, aX, aV, aF,
+        chained(k_adjG2P<Multi>, pg, kAdjThreads, 0, stream)(p, sc, sx, activeMask, sF, stride, shapeTable, sp, ts.gridV, aX, aV, aF,
                                                 aC, gridG, records);
-        k_accumulate<0, Multi><<<p2gCtas, 64, 0, stream>>>(p, sc, ts.hdr, ts.activeList, ts.blockEnd, ts.sortedIds,
-                                                            ts.cellStart, records, cutMasks, gridG, gridF);
-        k_adjGridUpdate<Multi><<<updCtas, 256, 0, stream>>>(p, sc, ts.hdr, ts.touchedList, shapeTable, sp, ts.gridA, gridG);
-        k_adjP2G<Multi><<<pg, kAdjThreads, 0, stream>>>(p, sc, sx, sv, activeMask, matParams, sF, sC, V0, stride, gridG, aX, aV,
+        chained(k_accumulate<0, Multi>, p2gCtas, 64, 0, stream)(p, sc, ts.hdr, ts.activeList, ts.blockEnd, ts.sortedIds,
+                                                            ts.cellStart, records, cutMasks, gridG, gridF, nullptr, nullptr);
+        chained(k_adjGridUpdate<Multi>, updCtas, 256, 0, stream)(p, sc, ts.hdr, ts.touchedList, shapeTable, sp, ts.gridA, gridG);
+        chained(k_adjP2G<Multi>, pg, kAdjThreads, 0, stream)(p, sc, sx, sv, activeMask, matParams, sF, sC, V0, stride, gridG, aX, aV,
                                                 aF, aC, aMat);
         CRB_LAUNCHED(4);
         return CRB200_OK;

@@ -41,7 +41,7 @@ namespace crb200
         int numShapes;
         unsigned particleBegin;
         int shapeBegin;
-        int pad;
+        int earlyNext; // small scene: the next kernel may come in early (chainStart)
     };
 
     // Scene lookup handed to every kernel.  With one scene the kernels use their StepParams

@@ -38,6 +38,17 @@ namespace crb200
     constexpr int kScanTile = 256; // blocks per scan tile
     constexpr int kScanThreads = 256;
 
+    // First statement of every kernel of a substep: nothing of it runs before the kernel ahead of it
+    // has completed and its writes are visible.  early: the kernel launched behind it may take its
+    // place on the SMs as soon as all of this one's CTAs have started, not only when they are done.
+    // (Both are no-ops in an ordinary launch.)
+    __device__ __forceinline__ void chainStart(int early = 0)
+    {
+        if (early)
+            cudaTriggerProgrammaticLaunchCompletion();
+        cudaGridDependencySynchronize();
+    }
+
     // ---------------------------------------------------------------------------------------
     // Addressing helpers
     __device__ __forceinline__ unsigned nodeAddr(const GridGeom &g, int i, int j, int k)
@@ -293,6 +304,7 @@ namespace crb200
                           unsigned *__restrict__ ranks, unsigned *__restrict__ blockCount,
                           unsigned *__restrict__ cellCount, unsigned *__restrict__ activeList, SortHeader *hdr)
     {
+        chainStart(p.earlyNext);
         if (honourSkip && hdr->sortSkip)
             return; // the resident path keeps its order this call
         const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -350,6 +362,7 @@ namespace crb200
                                                         unsigned *__restrict__ touchedFlag, unsigned *__restrict__ touchedList,
                                                         unsigned capacity, SortHeader *hdr)
     {
+        chainStart(p.earlyNext);
         if ((int)blockIdx.x < shapeCtas)
         {
             gatherSceneShapes(blockIdx.x, p, sc, shapeIds, shd, ge, shapeTable);
@@ -680,6 +693,7 @@ namespace crb200
                                                       const unsigned *__restrict__ cellStart,
                                                       unsigned *__restrict__ sortedIds)
     {
+        chainStart();
         __shared__ unsigned sIds[kCellOrderCap];
         const unsigned tid = threadIdx.x, nAct = hdr->numActiveBlocks;
         for (unsigned ab = blockIdx.x; ab < nAct; ab += gridDim.x)
@@ -843,6 +857,7 @@ namespace crb200
                                                         const unsigned char *__restrict__ blockFlags,
                                                         unsigned *__restrict__ touchedFlag)
     {
+        chainStart(p0.earlyNext);
         // touchedFlag: the block's "already listed" flag, cleared as it is consumed
         __shared__ ShapeRec sh[Multi ? 1 : kMaxShapes];
         __shared__ unsigned sTouched;
@@ -1009,6 +1024,7 @@ namespace crb200
                                                           const ShapeRec *__restrict__ shapeTable, int numShapes,
                                                           float4 *force, float4 *torque)
     {
+        chainStart();
         __shared__ float sSum[256][kDetSlots * 6 + 1];
         // word numMaskWords is set when any block holds partials (not on substeps without coupling)
         if (detMask[numMaskWords] == 0u)
@@ -1178,6 +1194,7 @@ namespace crb200
                                                  float4 *xo, float4 *vo, float *Fo, float *Co, bool lean,
                                                  unsigned *__restrict__ activeList)
     {
+        chainStart(p0.earlyNext);
         // Modes 0 and 2 write the updated state to xo, vo, Fo, Co: the input arrays themselves in an
         // ordinary substep, the next tape slot in the adjoint's replay (which keeps its input).
         // Inputs and outputs may therefore alias, so none of xm, vel, F, Cm, xo, vo, Fo, Co is
@@ -1472,6 +1489,7 @@ namespace crb200
                                                          SdfPtrs sdf, unsigned *status,
                                                          const unsigned long long *__restrict__ blockShapeMask)
     {
+        chainStart(p0.earlyNext);
         __shared__ ShapeRec sh[Multi ? 1 : kMaxShapes];
         if (!Multi && p0.numShapes > 0)
             loadShapes(sh, shapeTable, p0.numShapes);
@@ -1673,6 +1691,7 @@ namespace crb200
                                const unsigned char *__restrict__ mask, const ShapeRec *__restrict__ shapeTable,
                                SdfPtrs sdf, unsigned *__restrict__ out)
     {
+        chainStart(p0.earlyNext);
         __shared__ ShapeRec sh[Multi ? 1 : kMaxShapes];
         if (!Multi)
         {
@@ -1745,6 +1764,7 @@ namespace crb200
                                unsigned *__restrict__ tEnd, unsigned *__restrict__ tActive,
                                unsigned *__restrict__ tTouched, SortHeader *__restrict__ tHdr)
     {
+        chainStart();
         const unsigned stepN = gridDim.x * blockDim.x, i0 = blockIdx.x * blockDim.x + threadIdx.x;
         const unsigned nSorted = min(hdr->numSorted, n), nAct = hdr->numActiveBlocks, nT = hdr->numTouchedBlocks;
         for (unsigned i = i0; i < nSorted; i += stepN)
@@ -1838,6 +1858,44 @@ namespace crb200
         if (e_ != cudaSuccess)                              \
             return cudaFail(e_, "kernel launch");           \
     } while (0)
+
+    // A launch that may overlap its start with the end of the kernel before it in the stream
+    // (programmatic dependent launch; edges of that kind when captured).  Only for kernels that begin
+    // with chainStart(), every one of whose CTAs waits there: a chain of such kernels then completes
+    // in order.  It hides the start-up of a launch: 10 substeps of standard MPM at 64k particles 455 ->
+    // 440 us, 10 PB-MPM steps at 9k 2235 -> 2170 us, no difference at 1.6M.
+    //
+    // Single scenes of up to kEarlyParticles also let the next kernel's CTAs in while the last of
+    // theirs run: 4096 particles 291 -> 275 us, 13.8k 301 -> 287 us, PB-MPM at 16k 435 -> 422 us.
+    // Above, the CTAs that come early crowd on the SMs that happen to be free, and their kernel ends
+    // later: standard MPM at 33k 427 -> 551 us, PB-MPM at 37k 443 -> 465 us, batches alike.
+    constexpr unsigned kEarlyParticles = 24000;
+    template <class... P>
+    struct Chained
+    {
+        void (*kernel)(P...);
+        cudaLaunchConfig_t cfg;
+        template <class... A>
+        void operator()(A &&...args)
+        {
+            cudaLaunchAttribute at{};
+            at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            at.val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...); // an error is seen by CRB_LAUNCHED
+        }
+    };
+    template <class... P>
+    static Chained<P...> chained(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream)
+    {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(grid);
+        cfg.blockDim = dim3(block);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        return Chained<P...>{kernel, cfg};
+    }
 
     GridGeom makeGridGeom(float cellSize, const float mn[3], const float mx[3], unsigned blockBase)
     {
@@ -1936,7 +1994,7 @@ namespace crb200
             p.numShapes = d.numShapes;
             p.particleBegin = (unsigned)d.particleOffset;
             p.shapeBegin = d.shapeOffset;
-            p.pad = 0;
+            p.earlyNext = 0;
             out.push_back(p);
         }
         return out;
@@ -2071,7 +2129,7 @@ namespace crb200
         p.numShapes = numShapes;
         p.particleBegin = 0;
         p.shapeBegin = 0;
-        p.pad = 0;
+        p.earlyNext = !isBatch() && numActive <= kEarlyParticles ? 1 : 0;
         return p;
     }
 
@@ -2259,14 +2317,14 @@ namespace crb200
         {
             if (!carriedIn)
             {
-                k_bin<Multi><<<std::max(pg, 1u), 128, 0, stream>>>(p, sc, isStd, false, positionMass, activeMask, keys,
+                chained(k_bin<Multi>, std::max(pg, 1u), 128, 0, stream)(p, sc, isStd, false, positionMass, activeMask, keys,
                                                                    ranks, blockCount, cellCount, activeList, header);
                 CRB_LAUNCHED(1);
             }
             if (det2)
                 CRB_CHECK(cudaMemsetAsync(blockFlags, 0, totalBlocks, stream));
             const int shapeCtas = numShapes > 0 ? numScenes() : 0;
-            k_sortBlocks<<<shapeCtas + cellCtas, 256, 0, stream>>>(
+            chained(k_sortBlocks, shapeCtas + cellCtas, 256, 0, stream)(
                 p, sc, shapeCtas, shapeIds, shapes, geometries, shapeTable, activeList, blockCount, cellCount, cellStart,
                 blockEnd, det2 ? blockFlags : nullptr, touchedFlag, touchedList, (unsigned)numMaxParticles, header);
             CRB_LAUNCHED(1);
@@ -2275,7 +2333,7 @@ namespace crb200
         // iterations, so one evaluation serves every iteration; MLS-MPM's k_place evaluates them).
         if (numShapes > 0 && isPb && pg)
         {
-            k_cutMasks<Multi><<<std::min(pg, (unsigned)strideCtas), 128, 0, stream>>>(p, sc, positionMass, activeMask,
+            chained(k_cutMasks<Multi>, std::min(pg, (unsigned)strideCtas), 128, 0, stream)(p, sc, positionMass, activeMask,
                                                                                      shapeTable, sp, cutMasks);
             CRB_LAUNCHED(1);
         }
@@ -2286,7 +2344,7 @@ namespace crb200
             // (a scene without shapes has no slicer: no CTA more than placing needs)
             const unsigned per = M == 0 && !Multi && carriedIn && numShapes == 0 ? kPlacePer : 1u;
             const unsigned placeCtas = (nPart + kPlaceThreads * per - 1) / (kPlaceThreads * per);
-            k_place<M, Multi><<<placeCtas, kPlaceThreads, 0, stream>>>(
+            chained(k_place<M, Multi>, placeCtas, kPlaceThreads, 0, stream)(
                 p, sc, carriedIn, keys, ranks, cellStart, sortedIds, (unsigned)numMaxParticles, positionMass, velocity,
                 matParams, matType, F, Cm, V0, stride, shapeTable, sp, cutMasks, records, gridA, gridF,
                 &header->fp64Fallbacks);
@@ -2303,7 +2361,7 @@ namespace crb200
             return r;
         if (nPart > 0 && det2 && solves)
         {
-            k_cellOrder<<<cellCtas * 4, 64, 0, stream>>>(header, activeList, blockEnd, cellStart, sortedIds);
+            chained(k_cellOrder, cellCtas * 4, 64, 0, stream)(header, activeList, blockEnd, cellStart, sortedIds);
             CRB_LAUNCHED(1);
         }
         markPhase(1);
@@ -2312,12 +2370,12 @@ namespace crb200
             if (!pg)
                 return CRB200_OK;
             if (det2)
-                k_accumulate<M, Multi, true><<<p2gCtas, 64, 0, stream>>>(p, sc, header, activeList, blockEnd, sortedIds,
+                chained(k_accumulate<M, Multi, true>, p2gCtas, 64, 0, stream)(p, sc, header, activeList, blockEnd, sortedIds,
                                                                        cellStart, records, cutMasks, gridA, gridF,
                                                                        detTiles, detTilesF);
             else
-                k_accumulate<M, Multi><<<p2gCtas, 64, 0, stream>>>(p, sc, header, activeList, blockEnd, sortedIds,
-                                                                    cellStart, records, cutMasks, gridA, gridF);
+                chained(k_accumulate<M, Multi>, p2gCtas, 64, 0, stream)(p, sc, header, activeList, blockEnd, sortedIds,
+                                                                    cellStart, records, cutMasks, gridA, gridF, nullptr, nullptr);
             CRB_LAUNCHED(1);
             return CRB200_OK;
         };
@@ -2325,7 +2383,7 @@ namespace crb200
             const int det = detLevel(recompute || adjReplay);
             auto upd = [&](auto detTag) {
                 constexpr int D = decltype(detTag)::value;
-                k_gridUpdate<Multi, D><<<updCtas, 256, 0, stream>>>(
+                chained(k_gridUpdate<Multi, D>, updCtas, 256, 0, stream)(
                     p, sc, header, touchedList, shapeTable, sp, gridA, gridF, gridV, (recompute || adjReplay) ? adjForce : cf,
                     (recompute || adjReplay) ? adjTorque : ct, !recompute || tapeActive >= 0, blockShapeMask,
                     tapeActive >= 0 ? tapeSlot(tapeActive).gridA : nullptr,
@@ -2340,7 +2398,7 @@ namespace crb200
                         upd(std::integral_constant<int, 2>{});
                     else
                         upd(std::integral_constant<int, 1>{});
-                    k_coupleReduce<<<1, 256, 0, stream>>>((totalBlocks + 31) / 32, detMask, detPartials, shapeTable,
+                    chained(k_coupleReduce, 1, 256, 0, stream)((totalBlocks + 31) / 32, detMask, detPartials, shapeTable,
                                                           numShapes, (recompute || adjReplay) ? adjForce : cf,
                                                           (recompute || adjReplay) ? adjTorque : ct);
                     CRB_LAUNCHED(2);
@@ -2359,7 +2417,7 @@ namespace crb200
             if (tapeActive >= 0)
             {
                 const TapeSlot ts = tapeSlot(tapeActive);
-                k_tapeSort<<<strideCtas, 256, 0, stream>>>(totalParticles(), sortedIds, cellStart, blockEnd, activeList,
+                chained(k_tapeSort, strideCtas, 256, 0, stream)(totalParticles(), sortedIds, cellStart, blockEnd, activeList,
                                                           touchedList, header, ts.sortedIds, ts.cellStart, ts.blockEnd,
                                                           ts.activeList, ts.touchedList, ts.hdr);
                 CRB_LAUNCHED(1);
@@ -2372,7 +2430,7 @@ namespace crb200
             if (!pg)
                 return CRB200_OK;
             const unsigned char *g2pMask = (M == 2 && stdGpuSemantics && onesMask) ? onesMask : activeMask;
-            k_g2p<M, Multi><<<pg, 128, 0, stream>>>(p, sc, positionMass, velocity, g2pMask, F, Cm, stride, shapeTable,
+            chained(k_g2p<M, Multi>, pg, 128, 0, stream)(p, sc, positionMass, velocity, g2pMask, F, Cm, stride, shapeTable,
                                                     sp, gridV, cutMasks, &header->status, matParams, matType, V0,
                                                     ((M == 0 && carryOut) || (M == 1 && pbRecords)) ? records : nullptr,
                                                     gridA, header, keys, ranks, blockCount, cellCount, blockShapeMask,
@@ -2407,7 +2465,7 @@ namespace crb200
             }
             if (pg)
             {
-                k_pbIntegrate<Multi><<<pg, 128, 0, stream>>>(p, sc, positionMass, velocity, activeMask, F, Cm, stride,
+                chained(k_pbIntegrate<Multi>, pg, 128, 0, stream)(p, sc, positionMass, velocity, activeMask, F, Cm, stride,
                                                              shapeTable, sp, &header->status, blockShapeMask);
                 CRB_LAUNCHED(1);
             }

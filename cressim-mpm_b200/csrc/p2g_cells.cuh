@@ -313,6 +313,7 @@ namespace crb200
                                                     unsigned *__restrict__ cutMasks, float4 *__restrict__ records,
                                                     float4 *__restrict__ gridA, float4 *__restrict__ gridF, unsigned *fp64Count)
     {
+        chainStart(p0.earlyNext);
         const unsigned n = Multi ? sc.numParticles : p0.numActive;
         const bool anyCut = Mode == 0 && (Multi || p0.numShapes > 0) && (*sc.anyFlags & SF_SLICER);
         const bool cutScene = !Multi && anyCut;
@@ -408,6 +409,7 @@ namespace crb200
                                                        float4 *__restrict__ gridF, float4 *__restrict__ tiles = nullptr,
                                                        float4 *__restrict__ tilesF = nullptr)
     {
+        chainStart(p0.earlyNext);
         __shared__ unsigned sStart[65];
         __shared__ unsigned sOv[65];
         __shared__ unsigned sWarpTot;
