@@ -1089,8 +1089,7 @@ namespace crb200
         CRB_CHECK(cudaMemsetAsync(gridG, 0, (size_t)totalBlocks * 64 * sizeof(float4), stream));
         chained(k_adjG2P<Multi>, pg, kAdjThreads, 0, stream)(p, sc, sx, activeMask, sF, stride, shapeTable, sp, ts.gridV, aX, aV, aF,
                                                 aC, gridG, records);
-        chained(k_accumulate<0, Multi>, p2gCtas, 64, 0, stream)(p, sc, ts.hdr, ts.activeList, ts.blockEnd, ts.sortedIds,
-                                                            ts.cellStart, records, cutMasks, gridG, gridF, nullptr, nullptr);
+        launchAccumulate<0, Multi, false>(p, sc, ts.hdr, ts.activeList, ts.blockEnd, ts.cellStart, ts.sortedIds, gridG);
         chained(k_adjGridUpdate<Multi>, updCtas, 256, 0, stream)(p, sc, ts.hdr, ts.touchedList, shapeTable, sp, ts.gridA, gridG);
         chained(k_adjP2G<Multi>, pg, kAdjThreads, 0, stream)(p, sc, sx, sv, activeMask, matParams, sF, sC, V0, stride, gridG, aX, aV,
                                                 aF, aC, aMat);

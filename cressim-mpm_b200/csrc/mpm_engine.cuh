@@ -198,7 +198,7 @@ namespace crb200
         ShapeRec *shapeTable = nullptr;
         unsigned totalBlocks = 0;
         unsigned numTiles = 0;
-        int p2gCtas = 0;
+        int p2gCtas = 0, p2gPerSm = 1;
         int sortCtas = 0;
         int updCtas = 0;
         int strideCtas = 0;
@@ -223,6 +223,9 @@ namespace crb200
         int launchStep(bool carriedIn, bool carryOut); // enqueue one step's kernels
         template <bool Multi>
         int launchStepT(bool recompute, bool carriedIn, bool carryOut);
+        template <int Mode, bool Multi, bool Det>
+        void launchAccumulate(const StepParams &p, const SceneTable &sc, const SortHeader *hdr, const unsigned *active,
+                              const unsigned *ends, const unsigned *starts, const unsigned *ids, float4 *grid);
 
         // adjoint of the MLS-MPM substep (CrB200SolverAdjointRecord / AdjointBackward)
         int adjointRecord(int numSubsteps, int interval, const int *captures, int numCaptures, float4 *capturedX);

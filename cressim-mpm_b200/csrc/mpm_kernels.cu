@@ -2204,8 +2204,9 @@ namespace crb200
         int dev = 0, sms = 0, perSm = 0;
         CRB_CHECK(cudaGetDevice(&dev));
         CRB_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        CRB_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_accumulate<0, false>, 64, 0));
-        p2gCtas = sms * (perSm > 0 ? perSm : 1);
+        CRB_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_accumulate<0, false, false, 1>, 64, 0));
+        p2gPerSm = perSm > 0 ? perSm : 1;
+        p2gCtas = sms * p2gPerSm;
         sortCtas = sms * 4;  // 64-thread CTAs of the on-request sort-state kernel
         cellCtas = sms * 6;  // 256-thread CTAs of the sort (one warp per active block)
         updCtas = sms * 8;
@@ -2262,6 +2263,27 @@ namespace crb200
         if (isBatch())
             return launchStepT<true>(false, carriedIn, carryOut);
         return launchStepT<false>(false, carriedIn, carryOut);
+    }
+
+    // The cell accumulation of the given sort into `grid`, with as many threads per cell as the number
+    // of particles leaves room for (see k_accumulate).
+    template <int Mode, bool Multi, bool Det>
+    void Solver::launchAccumulate(const StepParams &p, const SceneTable &sc, const SortHeader *hdr, const unsigned *active,
+                                  const unsigned *ends, const unsigned *starts, const unsigned *ids, float4 *grid)
+    {
+        auto run = [&](auto split, unsigned ctas) {
+            constexpr int S = decltype(split)::value;
+            chained(k_accumulate<Mode, Multi, Det, S>, ctas, 64 * S, 0, stream)(
+                p, sc, hdr, active, ends, ids, starts, records, cutMasks, grid, gridF, Det ? detTiles : nullptr,
+                Det ? detTilesF : nullptr);
+        };
+        const unsigned n = sc.numParticles, each = (unsigned)std::max(p2gCtas / std::max(p2gPerSm, 1), 1); // CTAs / CTAs per SM
+        if (n <= (Multi ? kSplit4Batch : kSplit4))
+            run(std::integral_constant<int, 4>{}, each);
+        else if (n <= (Multi ? kSplit2Batch : kSplit2))
+            run(std::integral_constant<int, 2>{}, 3u * each);
+        else
+            run(std::integral_constant<int, 1>{}, (unsigned)p2gCtas);
     }
 
     // recompute: a forward substep up to the grid update only (the adjoint's replay of a segment's
@@ -2369,13 +2391,14 @@ namespace crb200
             constexpr int M = decltype(mode)::value;
             if (!pg)
                 return CRB200_OK;
+            auto run = [&](auto det) {
+                constexpr bool D = decltype(det)::value;
+                launchAccumulate<M, Multi, D>(p, sc, header, activeList, blockEnd, cellStart, sortedIds, gridA);
+            };
             if (det2)
-                chained(k_accumulate<M, Multi, true>, p2gCtas, 64, 0, stream)(p, sc, header, activeList, blockEnd, sortedIds,
-                                                                       cellStart, records, cutMasks, gridA, gridF,
-                                                                       detTiles, detTilesF);
+                run(std::true_type{});
             else
-                chained(k_accumulate<M, Multi>, p2gCtas, 64, 0, stream)(p, sc, header, activeList, blockEnd, sortedIds,
-                                                                    cellStart, records, cutMasks, gridA, gridF, nullptr, nullptr);
+                run(std::false_type{});
             CRB_LAUNCHED(1);
             return CRB200_OK;
         };

@@ -1,16 +1,17 @@
 // P2G with one thread per grid cell (included by mpm_kernels.cu).
 //
-// One 64-thread CTA takes one 4x4x4-cell block of the sorted particle list:
+// One CTA of 64 threads (128 or 256 in small scenes) takes one 4x4x4-cell block of the sorted
+// particle list:
 //   1. the block's cell ranges come from the per-cell starts of the sort;
-//   2. thread c walks the particles of cell c in sorted order, loading each one a particle ahead,
-//      turns it into the affine contribution u + i*a0 + j*a1 + k*a2 (MLS / PB-MPM) and
-//      accumulates the 27 stencil nodes in registers (the sums inside a block are deterministic);
+//   2. the threads of cell c walk its particles in sorted order, loading each one a particle ahead,
+//      turn it into the affine contribution u + i*a0 + j*a1 + k*a2 (MLS / PB-MPM) and
+//      accumulate the 27 stencil nodes in registers (the sums inside a block are deterministic);
 //   3. a 27-phase flush adds the registers into a per-warp shared-memory 6x6x6 node tile: in one
 //      phase the 32 lanes of a warp write 32 distinct nodes, so no atomics are needed;
-//   4. the two warp tiles are summed in a fixed order and each touched node gets one float4
+//   4. the warp tiles are summed in a fixed order and each touched node gets one float4
 //      vector atomic in the block-major accumulation grid.
 // Particles whose stencil base lies outside the grid take a per-particle path with global vector
-// atomics instead, and particles beyond the first kCellRun of a cell are added by vector atomics.
+// atomics instead, and particles beyond the first kCellRun of a thread are added by vector atomics.
 #pragma once
 
 namespace crb200
@@ -18,6 +19,9 @@ namespace crb200
     constexpr int kRec = 16;       // floats per staged particle
     constexpr int kCellRun = 9;    // particles a cell thread accumulates; the rest of a cell's
                                    // particles go through per-particle vector atomics
+
+    // Particles up to which a cell gets 4 threads, and 2 (see k_accumulate).
+    constexpr unsigned kSplit4 = 30000, kSplit2 = 100000, kSplit4Batch = 12000, kSplit2Batch = 48000;
 
     // Per-particle scatter with global vector atomics (outliers and oversized blocks).
     // Mode 0 MLS, 1 PB (u/a already include the mass), 2 standard momentum, 3 standard force.
@@ -398,30 +402,43 @@ namespace crb200
     //     (no kCellRun cap) and the block's whole 6x6x6 tile is stored to tiles[block] (tilesF for
     //     the standard solver's force pass), from which the grid update sums each node's sources in
     //     a fixed order.
-    template <int Mode, bool Multi, bool Det = false>
-    __global__ void __launch_bounds__(64, Multi ? 5 : 6) k_accumulate(const __grid_constant__ StepParams p0, SceneTable sc, const SortHeader *__restrict__ hdr,
+    //     Split: threads per cell.  Split threads take every Split-th particle of the cell, each with its
+    //     own node sums and its warp with its own tile.  With one thread per cell a block is a serial
+    //     walk of up to kCellRun particles, which is what the kernel costs while its blocks fit on the
+    //     SMs at once; more threads shorten the walk but take the SM's registers from other blocks (6,
+    //     3 and 1 CTAs fit).  10 substeps with 1 / 2 / 4 threads per cell, us: 4096 particles 270 / 238
+    //     / 233, 22k 292 / 270 / 256, 64k 312 / 292 / 330, 111k 338 / 335 / 396, 176k 437 / 460 / 521;
+    //     standard MPM 64k 453 / 434 / 475; a PB-MPM step at 98k 264 / 248 / 265, at 221k 361 / 377 /
+    //     431.  The lines below follow these at 8 particles per cell, with room for half as many; the
+    //     blocks of a batch are less full (12k 315 / 297 / 292, 40k 334 / 315 / 355, 70k 374 / 389 / 464).
+    template <int Mode, bool Multi, bool Det, int Split>
+    __global__ void __launch_bounds__(64 * Split, Split == 1 ? (Multi ? 5 : 6) : (Split == 2 ? 3 : 1)) k_accumulate(const __grid_constant__ StepParams p0, SceneTable sc, const SortHeader *__restrict__ hdr,
                                                        const unsigned *__restrict__ activeList,
                                                        const unsigned *__restrict__ blockEnd,
                                                        const unsigned *__restrict__ sortedIds,
                                                        const unsigned *__restrict__ cellStart,
                                                        const float4 *__restrict__ records,
                                                        const unsigned *__restrict__ cutMasks, float4 *__restrict__ gridA,
-                                                       float4 *__restrict__ gridF, float4 *__restrict__ tiles = nullptr,
-                                                       float4 *__restrict__ tilesF = nullptr)
+                                                       float4 *__restrict__ gridF, float4 *__restrict__ tiles,
+                                                       float4 *__restrict__ tilesF)
     {
         chainStart(p0.earlyNext);
         __shared__ unsigned sStart[65];
         __shared__ unsigned sOv[65];
         __shared__ unsigned sWarpTot;
-        __shared__ float sTile[2][4 * kTileNodes];
+        constexpr int kThreads = 64 * Split, kWarps = 2 * Split;
+        constexpr unsigned kRun = (unsigned)(kCellRun * Split); // particles of a cell its threads take
+        __shared__ float sTile[kWarps][4 * kTileNodes];
         __shared__ StepParams sP; // Multi: the current block's scene parameters
 
         const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+        const int cell = tid & 63; // the thread's cell; its particles are part, part + Split, ...
+        const unsigned part = (unsigned)tid >> 6;
         const int passes = Mode == 2 ? 2 : 1;
-        for (int t = tid; t < 2 * 4 * kTileNodes; t += 64)
+        for (int t = tid; t < kWarps * 4 * kTileNodes; t += kThreads)
             (&sTile[0][0])[t] = 0.f;
         const unsigned nAct = hdr->numActiveBlocks;
-        const int cx = tid & 3, cy = (tid >> 2) & 3, cz = tid >> 4;
+        const int cx = cell & 3, cy = (cell >> 2) & 3, cz = cell >> 4;
         for (unsigned ab = blockIdx.x; ab < nAct; ab += gridDim.x)
         {
             const unsigned b = activeList[ab];
@@ -443,33 +460,37 @@ namespace crb200
             const unsigned start = cellStart[b * 64u], cnt = blockEnd[b] - start;
             // cell ranges of this block's sorted slots (cells are contiguous, in cell order)
             {
-                const unsigned excl = cellStart[b * 64u + tid] - start;
-                const unsigned v = (tid < 63 ? cellStart[b * 64u + tid + 1] - start : cnt) - excl;
-                sStart[tid] = excl;
-                if (tid == 63)
-                    sStart[64] = cnt;
-                // overflow prefix: particles beyond the first kCellRun of each cell
-                const unsigned ov = v > (unsigned)kCellRun ? v - (unsigned)kCellRun : 0u;
-                unsigned oinc = ov;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1)
+                unsigned oinc = 0;
+                if (tid < 64)
                 {
-                    const unsigned y = __shfl_up_sync(0xffffffffu, oinc, o);
-                    if (lane >= o)
-                        oinc += y;
+                    const unsigned excl = cellStart[b * 64u + tid] - start;
+                    const unsigned v = (tid < 63 ? cellStart[b * 64u + tid + 1] - start : cnt) - excl;
+                    sStart[tid] = excl;
+                    if (tid == 63)
+                        sStart[64] = cnt;
+                    // overflow prefix: particles beyond the first kRun of each cell
+                    oinc = v > kRun ? v - kRun : 0u;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1)
+                    {
+                        const unsigned y = __shfl_up_sync(0xffffffffu, oinc, o);
+                        if (lane >= o)
+                            oinc += y;
+                    }
                 }
                 __syncthreads();
                 if (tid == 31)
                     sWarpTot = oinc;
                 __syncthreads();
-                sOv[tid + 1] = oinc + (warp ? sWarpTot : 0u);
+                if (tid < 64)
+                    sOv[tid + 1] = oinc + (warp ? sWarpTot : 0u);
                 if (tid == 0)
                     sOv[0] = 0;
             }
             __syncthreads();
-            const unsigned cs = sStart[tid], ce = sStart[tid + 1];
+            const unsigned cs = sStart[cell] + part, ce = sStart[cell + 1];
             // Det: a cell thread takes all of its cell's particles, so nothing goes through atomics
-            const unsigned runEnd = Det ? ce : min(ce, cs + (unsigned)kCellRun);
+            const unsigned runEnd = Det ? ce : min(ce, sStart[cell] + kRun);
             for (int pass = 0; pass < passes; ++pass)
             {
                 float acc[27][4];
@@ -485,22 +506,22 @@ namespace crb200
                 unsigned nid = cs < runEnd ? sortedIds[start + cs] : 0u;
                 if (cs < runEnd)
                     loadRecord(records, nid, nxt);
-                for (unsigned q = cs; q < runEnd; ++q)
+                for (unsigned q = cs; q < runEnd; q += Split)
                 {
                     float rec[kRec];
 #pragma unroll
                     for (int e = 0; e < kRec; ++e)
                         rec[e] = nxt[e];
                     const unsigned id = nid;
-                    if (q + 1 < runEnd)
+                    if (q + Split < runEnd)
                     {
-                        nid = sortedIds[start + q + 1];
+                        nid = sortedIds[start + q + Split];
                         loadRecord(records, nid, nxt);
                     }
-                    if (q + 2 < runEnd)
+                    if (q + 2 * Split < runEnd)
                     {
                         // the record after next into L1 (no registers held for it)
-                        const float4 *ahead = records + 4ull * sortedIds[start + q + 2];
+                        const float4 *ahead = records + 4ull * sortedIds[start + q + 2 * Split];
                         asm volatile("prefetch.global.L1 [%0];" ::"l"(ahead));
                         asm volatile("prefetch.global.L1 [%0];" ::"l"(ahead + 2));
                     }
@@ -529,18 +550,23 @@ namespace crb200
                         }
                 __syncthreads();
                 // fixed-order sum of the warp tiles, one vector atomic per touched node
-                for (int t = tid; t < kTileNodes; t += 64)
+                for (int t = tid; t < kTileNodes; t += kThreads)
                 {
-                    const float m = sTile[0][t] + sTile[1][t];
-                    const float px = sTile[0][kTileNodes + t] + sTile[1][kTileNodes + t];
-                    const float py = sTile[0][2 * kTileNodes + t] + sTile[1][2 * kTileNodes + t];
-                    const float pz = sTile[0][3 * kTileNodes + t] + sTile[1][3 * kTileNodes + t];
+                    float m = sTile[0][t], px = sTile[0][kTileNodes + t], py = sTile[0][2 * kTileNodes + t],
+                          pz = sTile[0][3 * kTileNodes + t];
 #pragma unroll
-                    for (int c = 0; c < 4; ++c)
+                    for (int w = 1; w < kWarps; ++w)
                     {
-                        sTile[0][c * kTileNodes + t] = 0.f;
-                        sTile[1][c * kTileNodes + t] = 0.f;
+                        m += sTile[w][t];
+                        px += sTile[w][kTileNodes + t];
+                        py += sTile[w][2 * kTileNodes + t];
+                        pz += sTile[w][3 * kTileNodes + t];
                     }
+#pragma unroll
+                    for (int w = 0; w < kWarps; ++w)
+#pragma unroll
+                        for (int c = 0; c < 4; ++c)
+                            sTile[w][c * kTileNodes + t] = 0.f;
                     if (Det)
                     {
                         float4 *dst = (Mode == 2 && pass == 1) ? tilesF : tiles;
@@ -560,9 +586,9 @@ namespace crb200
                     else if (m != 0.f || px != 0.f || py != 0.f || pz != 0.f)
                         atomicAdd(&gridA[a], make_float4(px, py, pz, m));
                 }
-                // particles beyond the first kCellRun of a cell: one per thread, vector atomics
+                // particles beyond the first kRun of a cell: one per thread, vector atomics
                 const unsigned total = Det ? 0u : sOv[64];
-                for (unsigned kk = tid; kk < total; kk += 64)
+                for (unsigned kk = tid; kk < total; kk += kThreads)
                 {
                     int lo = 0, hi = 63;
                     while (lo < hi)
@@ -573,7 +599,7 @@ namespace crb200
                         else
                             hi = mid - 1;
                     }
-                    const unsigned slot = start + sStart[lo] + (unsigned)kCellRun + (kk - sOv[lo]);
+                    const unsigned slot = start + sStart[lo] + kRun + (kk - sOv[lo]);
                     float rec[kRec];
                     const unsigned sid = sortedIds[slot];
                     loadRecord(records, sid, rec);

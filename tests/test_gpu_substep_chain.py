@@ -62,3 +62,20 @@ def test_batch_of_scenes_with_and_without_slicer():
     for s, sc in enumerate(parts):
         _check(b.scene_state(s, st), sc, 4)
     assert b.solver.grid_stats()["num_sorted"] == sum(int(sc.mask.sum()) for sc in parts)
+
+
+@pytest.mark.parametrize("cells,ppc", [(15, 8), (16, 8), (23, 8), (24, 8), (4, 40), (12, 40)])
+@pytest.mark.parametrize("solver", ["mls", "standard", "deterministic"])
+def test_threads_per_cell(cells, ppc, solver):
+    """Both sides of the particle counts at which a cell gets 4, 2 and 1 threads (27000 / 32768, 97336 /
+    110592), and cells fuller than the threads' runs."""
+    sc = scenes.cube_drop(side=cells * 0.02, cell=0.02, ppc=ppc,
+                          solver=scenes.SOLVER_STANDARD if solver == "standard" else scenes.SOLVER_MLS)
+    sc.pos_mass[:, 1] -= np.float32(0.5 - cells * 0.01 - 0.01)
+    sc.vel[:, :3] = (0.2, -1.0, 0.1)
+    g = cb.DeviceScene(sc, compute_initial=solver != "deterministic")
+    if solver == "deterministic":
+        g.solver.set_option(cb.OPT_DETERMINISTIC, 1)
+        g.compute_initial_data()
+    g.step(4)
+    _check(g.state(), sc, 4)
