@@ -385,11 +385,7 @@ namespace crb200
                     atomicAdd(&gridG[sa.addr(a, b, c)], make_float4(gVn.x, gVn.y, gVn.z, 0.f));
                 }
             }
-            float4 *out = records + 4ull * i;
-            out[0] = make_float4(rec[0], rec[1], rec[2], rec[3]);
-            out[1] = make_float4(rec[4], rec[5], rec[6], rec[7]);
-            out[2] = make_float4(rec[8], rec[9], rec[10], rec[11]);
-            out[3] = make_float4(rec[12], rec[13], rec[14], rec[15]);
+            storeRecord(records, i, rec);
         }
         aX[i] = make_float4(gx.x, gx.y, gx.z, 0.f);
 #pragma unroll

@@ -1,20 +1,24 @@
 // sm_100a kernels of the B200 MPM substep engine and the host Solver that launches them.
 //
 // One substep (MLS-MPM; the reference's GpuMlsMpmSolver::step, gpu_mls_mpm_solver.cu:102-109):
-//   1. gatherShapes   scene shapes -> compact table (shapes may change between substeps); with the
-//                     slicer cut masks on a side stream beside the sort chain
+//   1. gatherShapes   scene shapes -> compact table (shapes may change between substeps); a launch
+//                     of its own only where the previous grid update could not do it
 //   2. bin            per particle: cell key (block-major), rank among its cell's particles, cell
-//                     and block counts (warp-aggregated atomics); done by the previous G2P when
-//                     it can be
-//   3. scan           block offsets, active-block list, touched-block list (3 kernels), then the
-//                     absolute start of every cell of the active blocks
-//   4. scatter        particle ids into their cells' slots (cells contiguous in key order; arrival
-//                     order inside a cell; the canonical order is produced on request)
-//   5. p2g            one CTA per active block: particles -> shared-memory 6x6x6 node tile ->
-//                     one float4 vector atomic per touched node into the accumulation grid
+//                     and block counts (warp-aggregated atomics), and the list of active blocks;
+//                     done by the previous G2P when it can be
+//   3. sortBlocks     over the listed blocks only: the start of every cell, the work items of the
+//                     accumulation and the list of touched blocks
+//   4. place          particle ids into their cells' slots (cells contiguous in key order; arrival
+//                     order inside a cell; the canonical order is produced on request), and the
+//                     P2G records and cut masks that the previous G2P did not leave
+//   5. accumulate     one CTA per work item: particles -> shared-memory 6x6x6 node tile -> one
+//                     float4 vector atomic per touched node into the accumulation grid
 //   6. gridUpdate     touched blocks only: momentum -> velocity, SDF contact/friction, domain BC,
 //                     and the accumulation grid is zeroed as it is consumed
-//   7. g2p            particle order: 27-node gather, APIC matrix, advection, push-out, F update
+//   7. g2p            particle order: 27-node gather, APIC matrix, advection, push-out, F update,
+//                     and the next substep's record and binning
+// The launches are a dependent chain (chainStart).  Deterministic substeps and the cell-ordered
+// path sort by block in an order that does not depend on arrival: bin, scan (3 kernels), scatter.
 // PB-MPM runs 6-8 `iterations` times per step plus an integration kernel (gpu_pb_mpm_solver.cu:
 // 102-113); standard MPM carries a node force tile (gpu_standard_mpm_solver.cu:177-184).
 
@@ -1402,7 +1406,7 @@ namespace crb200
                     for (int e = 0; e < kRec; ++e)
                         rec[e] = 0.f;
                 }
-                storeRecord(records + 4ull * i, rec);
+                storeRecord(records, i, rec);
             }
             return;
         }
@@ -1455,11 +1459,7 @@ namespace crb200
                 for (int e = 0; e < kRec; ++e)
                     rec[e] = 0.f;
             }
-            float4 *out = records + 4ull * i;
-            out[0] = make_float4(rec[0], rec[1], rec[2], rec[3]);
-            out[1] = make_float4(rec[4], rec[5], rec[6], rec[7]);
-            out[2] = make_float4(rec[8], rec[9], rec[10], rec[11]);
-            out[3] = make_float4(rec[12], rec[13], rec[14], rec[15]);
+            storeRecord(records, i, rec);
         }
         if (carry)
         {
@@ -2190,7 +2190,7 @@ namespace crb200
             CRB_CHECK(cudaMemcpy(dParams, ps.data(), ps.size() * sizeof(StepParams), cudaMemcpyHostToDevice));
         }
         CRB_CHECK(cudaMalloc(&cutMasks, n * sizeof(unsigned)));
-        CRB_CHECK(cudaMalloc(&records, n * 4 * sizeof(float4)));
+        CRB_CHECK(cudaMalloc(&records, (n + kRecTile - 1) / kRecTile * kRecTile * 4 * sizeof(float4)));
         CRB_CHECK(cudaMemsetAsync(F, 0, 9 * n * sizeof(float), stream));
         CRB_CHECK(cudaMemsetAsync(Cm, 0, 9 * n * sizeof(float), stream));
         CRB_CHECK(cudaMemsetAsync(V0, 0, n * sizeof(float), stream));
