@@ -52,7 +52,7 @@ namespace crb200
         const unsigned short *particleScene; // scene of each particle (0xFFFF: none)
         const unsigned short *blockScene;    // scene of each grid block
         unsigned *flags;                     // SF_* shape flags per scene
-        unsigned *anyFlags;                  // those of all scenes together
+        unsigned *anyFlags;                  // those of all scenes together (without a batch the same word)
         int numScenes;
         unsigned numParticles;               // particles covered by all scenes
     };

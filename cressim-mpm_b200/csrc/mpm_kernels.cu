@@ -287,7 +287,7 @@ namespace crb200
         if (threadIdx.x == 0)
         {
             sc.flags[scene] = (unsigned)flags;
-            if (sc.numScenes > 1 && flags)
+            if (sc.anyFlags != sc.flags && flags) // a batch, of one scene too
                 atomicOr(sc.anyFlags, (unsigned)flags); // zeroed with the counts of the sort
         }
     }
