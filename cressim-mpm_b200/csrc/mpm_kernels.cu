@@ -2190,6 +2190,7 @@ namespace crb200
             CRB_CHECK(cudaMemcpy(dParams, ps.data(), ps.size() * sizeof(StepParams), cudaMemcpyHostToDevice));
         }
         CRB_CHECK(cudaMalloc(&cutMasks, n * sizeof(unsigned)));
+        CRB_CHECK(cudaMemsetAsync(cutMasks, 0, n * sizeof(unsigned), stream));
         CRB_CHECK(cudaMalloc(&records, (n + kRecTile - 1) / kRecTile * kRecTile * 4 * sizeof(float4)));
         CRB_CHECK(cudaMemsetAsync(F, 0, 9 * n * sizeof(float), stream));
         CRB_CHECK(cudaMemsetAsync(Cm, 0, 9 * n * sizeof(float), stream));

@@ -363,8 +363,15 @@ namespace crb200
             __syncthreads();
         }
         const unsigned id = i0;
+        // The masks are handed out (CrB200SolverCopyCutMasks): zero for a particle that takes no part, and
+        // in a batch, whose masks are copied whole, for a scene without a slicer (once per call).
+        const bool handsOut = Mode == 0 && (Multi ? p0.numShapes > 0 : cutScene);
         if (key[0] == kInvalidKey)
+        {
+            if (handsOut && id < n)
+                cutMasks[id] = 0u;
             return;
+        }
         const unsigned si = Multi ? sc.particleScene[id] : 0u; // sorted particles have a scene
         const StepParams &p = Multi ? sc.params[si] : p0;
         const bool slicers = Mode <= 1 && p.numShapes > 0 && (sc.flags[si] & SF_SLICER);
@@ -382,6 +389,8 @@ namespace crb200
             else
                 msk = cutMasks[id];
         }
+        else if (Multi && handsOut)
+            cutMasks[id] = 0u;
         RawParticle raw;
         loadRaw<Mode>(id, xm, vel, matParams, matType, F, Cm, V0, stride, raw);
         float rec[kRec];
