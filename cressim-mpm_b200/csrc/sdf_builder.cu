@@ -259,15 +259,17 @@ namespace crb200
                         const float ax = A.x - q.x, ay = A.y - q.y, az = A.z - q.z;
                         const float bx = B.x - q.x, by = B.y - q.y, bz = B.z - q.z;
                         const float cx = Cc.x - q.x, cy = Cc.y - q.y, cz = Cc.z - q.z;
-                        const float la = fastLen(ax * ax + ay * ay + az * az);
-                        const float lb = fastLen(bx * bx + by * by + bz * bz);
-                        const float lc = fastLen(cx * cx + cy * cy + cz * cz);
+                        // inverse lengths: the term is taken of the unit vectors to the corners, so that
+                        // it and its square stay within a few units at any scale of the mesh
+                        const float ia = rsqrtf(ax * ax + ay * ay + az * az);
+                        const float ib = rsqrtf(bx * bx + by * by + bz * bz);
+                        const float ic = rsqrtf(cx * cx + cy * cy + cz * cz);
                         // the triple product of the corners is the plane's distance times |N|
-                        const float det = (N.x * ax + N.y * ay + N.z * az) * fabsf(N.w);
-                        const float den = la * lb * lc + (ax * bx + ay * by + az * bz) * lc +
-                                          (bx * cx + by * cy + bz * cz) * la + (cx * ax + cy * ay + cz * az) * lb;
+                        const float det = ((N.x * ax + N.y * ay + N.z * az) * ia) * (fabsf(N.w) * ib * ic);
+                        const float den = 1.f + (ax * bx + ay * by + az * bz) * ia * ib +
+                                          (bx * cx + by * cy + bz * cz) * ib * ic + (cx * ax + cy * ay + cz * az) * ic * ia;
                         // turn (wr, wi) by the angle of (den, det), which is at most pi either way, and
-                        // scale it back to unit length
+                        // scale it back to unit length (a corner at q has no angle: not a number here)
                         const float nr = wr * den - wi * det, ni = wr * det + wi * den;
                         const float m2 = nr * nr + ni * ni;
                         if (m2 > 0.f)
