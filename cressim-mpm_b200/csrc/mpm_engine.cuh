@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "../../include/crmpm_b200.h"
+#include "device_scope.cuh"
 #include "mpm_device.cuh"
 
 namespace crb200
@@ -161,6 +162,7 @@ namespace crb200
         int markPhase(int k); // record event k when phase timing is on
 
         bool initialized = false;
+        int device = 0; // where the solver's buffers and its stream are (initialize)
         unsigned configVersion = 0; // bumped by every setter so captured graphs are refreshed
 
         // solver-owned device state

@@ -2202,9 +2202,9 @@ namespace crb200
         CRB_CHECK(cudaMemsetAsync(blockCount, 0, (totalBlocks + 1) * sizeof(unsigned), stream));
         CRB_CHECK(cudaMemsetAsync(header, 0, sizeof(SortHeader), stream));
         CRB_CHECK(cudaMemsetAsync(keys, 0xff, n * sizeof(unsigned), stream));
-        int dev = 0, sms = 0, perSm = 0;
-        CRB_CHECK(cudaGetDevice(&dev));
-        CRB_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        int sms = 0, perSm = 0;
+        CRB_CHECK(cudaGetDevice(&device));
+        CRB_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
         CRB_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_accumulate<0, false, false, 1>, 64, 0));
         p2gPerSm = perSm > 0 ? perSm : 1;
         p2gCtas = sms * p2gPerSm;
@@ -3010,24 +3010,6 @@ namespace crb200
         }
     }
 
-    // Whether a kernel on this device can take `p` as an array of floats: memory of this device,
-    // managed or registered host memory, aligned to a float.  What it cannot take (another
-    // device's memory, odd addresses) goes through the copy engine.
-    static bool kernelReachable(const void *p)
-    {
-        if (reinterpret_cast<uintptr_t>(p) & 3u)
-            return false;
-        cudaPointerAttributes a{};
-        int dev = 0;
-        if (cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess)
-        {
-            cudaGetLastError(); // an unknown pointer is not an error of this call
-            return false;
-        }
-        return a.type == cudaMemoryTypeManaged || (a.type == cudaMemoryTypeHost && a.devicePointer == p) ||
-               (a.type == cudaMemoryTypeDevice && a.device == dev);
-    }
-
     // F and C (either may be null) of particles 0..n-1 between row arrays and the planes.
     template <bool ToPlanes>
     int Solver::moveMatrices(unsigned n, float *rowsF, float *rowsC)
@@ -3042,6 +3024,7 @@ namespace crb200
         auto flush = [&]() -> int {
             if (parts == 0)
                 return CRB200_OK;
+            const DeviceScope scope(device); // the caller may have another device current
             k_moveMatrices<ToPlanes><<<dim3((n + kMoveTile - 1) / kMoveTile, parts), kMoveTile, 0, stream>>>(
                 n, (unsigned)stride, mv);
             parts = 0;
@@ -3052,7 +3035,7 @@ namespace crb200
         {
             if (!rows[m])
                 continue;
-            if (kernelReachable(rows[m]))
+            if (kernelReachable(rows[m], (size_t)n * 9, device))
             {
                 mv.rows[parts] = rows[m];
                 mv.planes[parts++] = planes[m];
