@@ -2274,7 +2274,7 @@ namespace crb200
     {
         auto run = [&](auto split, unsigned ctas) {
             constexpr int S = decltype(split)::value;
-            chained(k_accumulate<Mode, Multi, Det, S>, ctas, 64 * S, 0, stream)(
+            chained(k_accumulate<Mode, Multi, Det, S>, ctas, 64 * kGroups<Mode, S>, 0, stream)(
                 p, sc, hdr, active, ends, ids, starts, records, cutMasks, grid, gridF, Det ? detTiles : nullptr,
                 Det ? detTilesF : nullptr);
         };

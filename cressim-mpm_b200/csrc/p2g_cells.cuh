@@ -1,6 +1,6 @@
 // P2G with one thread per grid cell (included by mpm_kernels.cu).
 //
-// One CTA of 64 threads (128 or 256 in small scenes) takes one 4x4x4-cell block of the sorted
+// 64 threads (128 or 256 in small scenes of few blocks) take one 4x4x4-cell block of the sorted
 // particle list:
 //   1. the block's cell ranges come from the per-cell starts of the sort;
 //   2. the threads of cell c walk its particles in sorted order, loading each one a particle ahead,
@@ -413,56 +413,68 @@ namespace crb200
         rec[12] = d.x; rec[13] = d.y; rec[14] = d.z; rec[15] = d.w;
     }
 
-    // (c) Cell accumulation: one 64-thread CTA per active block, one thread per cell.
-    //     Multi: each active block reads its scene's parameters.
-    //     Det: nothing is added atomically.  A cell thread accumulates all of its cell's particles
-    //     (no kCellRun cap) and the block's whole 6x6x6 tile is stored to tiles[block] (tilesF for
-    //     the standard solver's force pass), from which the grid update sums each node's sources in
-    //     a fixed order.
-    //     Split: threads per cell.  Split threads take every Split-th particle of the cell, each with its
-    //     own node sums and its warp with its own tile.  With one thread per cell a block is a serial
-    //     walk of up to kCellRun particles, which is what the kernel costs while its blocks fit on the
-    //     SMs at once; more threads shorten the walk but take the SM's registers from other blocks (6,
-    //     3 and 1 CTAs fit).  10 substeps with 1 / 2 / 4 threads per cell, us: 4096 particles 270 / 238
-    //     / 233, 22k 292 / 270 / 256, 64k 312 / 292 / 330, 111k 338 / 335 / 396, 176k 437 / 460 / 521;
-    //     standard MPM 64k 453 / 434 / 475; a PB-MPM step at 98k 264 / 248 / 265, at 221k 361 / 377 /
-    //     431.  The lines below follow these at 8 particles per cell, with room for half as many; the
-    //     blocks of a batch are less full (12k 315 / 297 / 292, 40k 334 / 315 / 355, 70k 374 / 389 / 464).
-    template <int Mode, bool Multi, bool Det, int Split>
-    __global__ void __launch_bounds__(64 * Split, Split == 1 ? (Multi ? 5 : 6) : (Split == 2 ? 3 : 1)) k_accumulate(const __grid_constant__ StepParams p0, SceneTable sc, const SortHeader *__restrict__ hdr,
-                                                       const unsigned *__restrict__ activeList,
-                                                       const unsigned *__restrict__ blockEnd,
-                                                       const unsigned *__restrict__ sortedIds,
-                                                       const unsigned *__restrict__ cellStart,
-                                                       const float4 *__restrict__ records,
-                                                       const unsigned *__restrict__ cutMasks, float4 *__restrict__ gridA,
-                                                       float4 *__restrict__ gridF, float4 *__restrict__ tiles,
-                                                       float4 *__restrict__ tilesF)
+    // Groups of 64 threads in a CTA of the cell accumulation (see k_accumulate).
+    template <int Mode, int Split>
+    constexpr int kGroups = Split == 4 ? 6 : Split;
+
+    // Shared memory of a CTA of the cell accumulation, whose groups may each have a block of their own.
+    template <int Mode, bool Multi, int Split>
+    struct AccumulateShared
     {
-        chainStart(p0.earlyNext);
-        __shared__ unsigned sStart[65];
-        __shared__ unsigned sOv[65];
-        __shared__ unsigned sWarpTot;
-        constexpr int kThreads = 64 * Split, kWarps = 2 * Split;
-        constexpr unsigned kRun = (unsigned)(kCellRun * Split); // particles of a cell its threads take
+        static constexpr int kWarps = 2 * kGroups<Mode, Split>;
         // Node tile of each warp: momentum and mass of node (x, y, z) at x + kPitch (y + 6 z).  With a
         // pitch of 12 the 8 lanes of a 16-byte access (4 cells in x, 2 in y) cover all bank groups;
-        // the widest CTAs, with 8 tiles, would pass 48 KB and take two-way conflicts.  One array of
+        // the widest CTAs, with 8 or 12 tiles, would pass 48 KB and take two-way conflicts.  One array of
         // float4 instead of four of floats: a quarter of the flush's instructions; a substep of
         // 1.6M particles 212 -> 209 us, of 85k 31.3 -> 31.1 us.
-        constexpr int kPitch = Split <= 2 ? 12 : kTileEdge, kTileSlots = kPitch * kTileEdge * kTileEdge;
-        __shared__ float4 sTile[kWarps][kTileSlots];
-        __shared__ StepParams sP; // Multi: the current block's scene parameters
+        static constexpr int kPitch = Split <= 2 ? 12 : kTileEdge, kTileSlots = kPitch * kTileEdge * kTileEdge;
+        float4 tile[kWarps][kTileSlots];
+        unsigned start[kGroups<Mode, Split>][65];
+        unsigned ov[kGroups<Mode, Split>][65];
+        unsigned warpTot[kGroups<Mode, Split>];
+        StepParams p[Multi ? kGroups<Mode, Split> : 1]; // Multi: the current block's scene parameters
+    };
 
-        const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-        const int cell = tid & 63; // the thread's cell; its particles are part, part + Split, ...
+    // The active blocks of a CTA, each worked on by a team of Step groups: Split groups, all on one block at a
+    // time, or single groups with blocks of their own.
+    template <int Mode, bool Multi, bool Det, int Split, int Step>
+    __device__ __forceinline__ void accumulateBlocks(AccumulateShared<Mode, Multi, Split> &sh, const StepParams &p0,
+                                                     const SceneTable &sc, unsigned nAct,
+                                                     const unsigned *__restrict__ activeList,
+                                                     const unsigned *__restrict__ blockEnd,
+                                                     const unsigned *__restrict__ sortedIds,
+                                                     const unsigned *__restrict__ cellStart,
+                                                     const float4 *__restrict__ records,
+                                                     const unsigned *__restrict__ cutMasks, float4 *__restrict__ gridA,
+                                                     float4 *__restrict__ gridF, float4 *__restrict__ tiles,
+                                                     float4 *__restrict__ tilesF)
+    {
+        constexpr bool kWhole = Step == Split; // one team; groups past it have nothing to do
+        constexpr int kThreads = 64 * Step, kWarps = 2 * Step;
+        constexpr unsigned kRun = (unsigned)(kCellRun * Step); // particles of a cell its threads take
+        constexpr int kPitch = AccumulateShared<Mode, Multi, Split>::kPitch, kTileSlots = AccumulateShared<Mode, Multi, Split>::kTileSlots;
+        if (kWhole && threadIdx.x >= (unsigned)kThreads)
+            return;
+        const unsigned team = kWhole ? 0u : threadIdx.x >> 6;
+        const int tid = (int)(threadIdx.x - 64u * team), lane = tid & 31, warp = tid >> 5; // within the team
+        const int cell = tid & 63; // the thread's cell; its particles are part, part + Step, ...
         const unsigned part = (unsigned)tid >> 6;
+        unsigned *sStart = sh.start[team], *sOv = sh.ov[team];
+        unsigned &sWarpTot = sh.warpTot[team];
+        StepParams &sP = sh.p[Multi ? team : 0u];
+        float4(*teamTile)[kTileSlots] = sh.tile + 2 * team;
+        auto teamSync = [&]() {
+            if constexpr (Split == 1)
+                __syncthreads();
+            else
+                asm volatile("bar.sync %0, %1;" ::"r"(kWhole ? 0u : 1u + team), "n"(kThreads) : "memory");
+        };
+        // A record is loaded into registers while its predecessor is worked on, but for standard MPM with more
+        // than one thread per cell: its second pass would spill (64k particles, 10 substeps 394 -> 384 us).
+        constexpr bool kAhead = !(Mode == 2 && Split > 1);
         const int passes = Mode == 2 ? 2 : 1;
-        for (int t = tid; t < kWarps * kTileSlots; t += kThreads)
-            (&sTile[0][0])[t] = make_float4(0.f, 0.f, 0.f, 0.f);
-        const unsigned nAct = hdr->numActiveBlocks;
         const int cx = cell & 3, cy = (cell >> 2) & 3, cz = cell >> 4;
-        for (unsigned ab = blockIdx.x; ab < nAct; ab += gridDim.x)
+        for (unsigned ab = blockIdx.x + team * gridDim.x; ab < nAct; ab += gridDim.x * (kWhole ? 1u : (unsigned)kGroups<Mode, Split>))
         {
             const unsigned b = activeList[ab];
             const unsigned si = Multi ? (unsigned)sceneOfBlock(sc, b) : 0u;
@@ -473,7 +485,7 @@ namespace crb200
                 static_assert(words <= 64, "StepParams must fit one load per thread");
                 if (tid < words)
                     reinterpret_cast<unsigned *>(&sP)[tid] = reinterpret_cast<const unsigned *>(&sc.params[si])[tid];
-                __syncthreads();
+                teamSync();
             }
             const StepParams &p = Multi ? sP : p0;
             const GridGeom &g = p.g;
@@ -501,16 +513,16 @@ namespace crb200
                             oinc += y;
                     }
                 }
-                __syncthreads();
+                teamSync();
                 if (tid == 31)
                     sWarpTot = oinc;
-                __syncthreads();
+                teamSync();
                 if (tid < 64)
                     sOv[tid + 1] = oinc + (warp ? sWarpTot : 0u);
                 if (tid == 0)
                     sOv[0] = 0;
             }
-            __syncthreads();
+            teamSync();
             const unsigned cs = sStart[cell] + part, ce = sStart[cell + 1];
             // Det: a cell thread takes all of its cell's particles, so nothing goes through atomics
             const unsigned runEnd = Det ? ce : min(ce, sStart[cell] + kRun);
@@ -527,24 +539,36 @@ namespace crb200
                 }
                 float nxt[kRec];
                 unsigned nid = cs < runEnd ? sortedIds[start + cs] : 0u;
-                if (cs < runEnd)
+                if (kAhead && cs < runEnd)
                     loadRecord(records, nid, nxt);
-                for (unsigned q = cs; q < runEnd; q += Split)
+                for (unsigned q = cs; q < runEnd; q += Step)
                 {
                     float rec[kRec];
-#pragma unroll
-                    for (int e = 0; e < kRec; ++e)
-                        rec[e] = nxt[e];
-                    const unsigned id = nid;
-                    if (q + Split < runEnd)
+                    if (!kAhead)
+                        loadRecord(records, nid, rec);
+                    else
                     {
-                        nid = sortedIds[start + q + Split];
-                        loadRecord(records, nid, nxt);
+#pragma unroll
+                        for (int e = 0; e < kRec; ++e)
+                            rec[e] = nxt[e];
                     }
-                    if (q + 2 * Split < runEnd)
+                    const unsigned id = nid;
+                    if (q + Step < runEnd)
+                    {
+                        nid = sortedIds[start + q + Step];
+                        if (kAhead)
+                            loadRecord(records, nid, nxt);
+                        else
+                        {
+                            const float4 *ahead = records + recordAt(nid);
+                            asm volatile("prefetch.global.L1 [%0];" ::"l"(ahead));
+                            asm volatile("prefetch.global.L1 [%0];" ::"l"(ahead + kRecHalf));
+                        }
+                    }
+                    if (kAhead && q + 2 * Step < runEnd)
                     {
                         // the record after next into L1 (no registers held for it)
-                        const float4 *ahead = records + recordAt(sortedIds[start + q + 2 * Split]);
+                        const float4 *ahead = records + recordAt(sortedIds[start + q + 2 * Step]);
                         asm volatile("prefetch.global.L1 [%0];" ::"l"(ahead));
                         asm volatile("prefetch.global.L1 [%0];" ::"l"(ahead + kRecHalf));
                     }
@@ -555,7 +579,7 @@ namespace crb200
                         accumulateCell<Mode, false>(p, rec, 0u, pass, acc);
                 }
                 // phased flush of the registers into this warp's tile
-                float4 *tile = sTile[warp] + cx + kPitch * (cy + kTileEdge * cz);
+                float4 *tile = teamTile[warp] + cx + kPitch * (cy + kTileEdge * cz);
 #pragma unroll
                 for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -573,19 +597,19 @@ namespace crb200
                             *t = v;
                             __syncwarp();
                         }
-                __syncthreads();
+                teamSync();
                 // fixed-order sum of the warp tiles, one vector atomic per touched node
                 for (int t = tid; t < kTileNodes; t += kThreads)
                 {
                     const int tx = t % kTileEdge, tyz = t / kTileEdge;
                     const int e = tx + kPitch * tyz;
-                    float4 v = sTile[0][e];
-                    sTile[0][e] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    float4 v = teamTile[0][e];
+                    teamTile[0][e] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                     for (int w = 1; w < kWarps; ++w)
                     {
-                        const float4 o = sTile[w][e];
-                        sTile[w][e] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        const float4 o = teamTile[w][e];
+                        teamTile[w][e] = make_float4(0.f, 0.f, 0.f, 0.f);
                         v = make_float4(v.x + o.x, v.y + o.y, v.z + o.z, v.w + o.w);
                     }
                     if (Det)
@@ -639,8 +663,58 @@ namespace crb200
                     else
                         scatterGlobal<Mode>(p, st, rec, msk, gridA, gridF);
                 }
-                __syncthreads();
+                teamSync();
             }
         }
+    }
+
+    // (c) Cell accumulation: groups of 64 threads, one thread per cell of an active block.
+    //     Multi: each active block reads its scene's parameters.
+    //     Det: nothing is added atomically.  A cell's threads accumulate all of its particles
+    //     (no kCellRun cap) and the block's whole 6x6x6 tile is stored to tiles[block] (tilesF for
+    //     the standard solver's force pass), from which the grid update sums each node's sources in
+    //     a fixed order.
+    //     Split: threads per cell, 1, 2 or 4 by the number of particles.  They take every Split-th particle
+    //     of the cell, each with its own node sums and its warp with its own tile.  With one thread per cell
+    //     a block is a serial walk of up to kCellRun particles, which is what the kernel costs while its
+    //     blocks fit on the SMs at once; more threads shorten the walk but take the SM's registers from
+    //     other blocks: 6, 3 and 1 blocks per SM are then worked on.  10 substeps with 1 / 2 / 4 threads
+    //     per cell, us: 4096 particles 270 / 238 / 233, 22k 292 / 270 / 256, 64k 312 / 292 / 330, 111k
+    //     338 / 335 / 396, 176k 437 / 460 / 521; standard MPM 64k 453 / 434 / 475; a PB-MPM step at 98k
+    //     264 / 248 / 265, at 221k 361 / 377 / 431.  The lines (kSplit4 and so on) follow these at 8 particles
+    //     per cell, with room for half as many; the blocks of a batch are less full (12k 315 / 297 /
+    //     292, 40k 334 / 315 / 355, 70k 374 / 389 / 464).
+    //     How many blocks that many particles lie in is known here only.  Where they are more than the CTAs
+    //     (the resident ones: one round of them), the groups of a CTA take blocks of their own, one thread
+    //     per cell, so that as many blocks are worked on as with 64-thread CTAs: 6 per SM with 2 threads
+    //     per cell and, for the sake of this, 6 groups in the CTAs with 4.  10 substeps, us, all groups on
+    //     one block -> on their own: 27k particles in 716 blocks 396 -> 273, PB-MPM 1585 -> 990, standard
+    //     576 -> 372; 29k strewn over 6000 blocks 1714 -> 671, PB-MPM 8041 -> 2830, standard 2965 -> 1146;
+    //     88k in 511 blocks 345 -> 334, PB-MPM 1344 -> 1332, standard 516 -> 518 (and 93k in 996, a last
+    //     round of few blocks, 390 -> 368, 1558 -> 1484 and 586 -> 603).
+    template <int Mode, bool Multi, bool Det, int Split>
+    __global__ void __launch_bounds__(64 * kGroups<Mode, Split>, Split == 1 ? (Multi ? 5 : 6) : (Split == 2 ? 3 : 1)) k_accumulate(const __grid_constant__ StepParams p0, SceneTable sc, const SortHeader *__restrict__ hdr,
+                                                       const unsigned *__restrict__ activeList,
+                                                       const unsigned *__restrict__ blockEnd,
+                                                       const unsigned *__restrict__ sortedIds,
+                                                       const unsigned *__restrict__ cellStart,
+                                                       const float4 *__restrict__ records,
+                                                       const unsigned *__restrict__ cutMasks, float4 *__restrict__ gridA,
+                                                       float4 *__restrict__ gridF, float4 *__restrict__ tiles,
+                                                       float4 *__restrict__ tilesF)
+    {
+        chainStart(p0.earlyNext);
+        __shared__ AccumulateShared<Mode, Multi, Split> sh;
+        const unsigned nAct = hdr->numActiveBlocks;
+        // each warp clears its own tile while the number of blocks is on its way
+        for (int t = threadIdx.x & 31; t < sh.kTileSlots; t += 32)
+            sh.tile[threadIdx.x >> 5][t] = make_float4(0.f, 0.f, 0.f, 0.f);
+        __syncwarp();
+        if (Split == 1 || nAct <= gridDim.x)
+            accumulateBlocks<Mode, Multi, Det, Split, Split>(sh, p0, sc, nAct, activeList, blockEnd, sortedIds, cellStart, records,
+                                                             cutMasks, gridA, gridF, tiles, tilesF);
+        else
+            accumulateBlocks<Mode, Multi, Det, Split, 1>(sh, p0, sc, nAct, activeList, blockEnd, sortedIds, cellStart, records,
+                                                         cutMasks, gridA, gridF, tiles, tilesF);
     }
 } // namespace crb200
