@@ -2873,8 +2873,9 @@ namespace crb200
                         cellCtas = baseSort * mul[c];
                     }
                     configVersion++;
-                    if ((r = loadState(snap)) != CRB200_OK || (r = stepMany(2)) != CRB200_OK)
-                        break; // builds the graph
+                    // every graph of the trial is captured before it is timed: a first, a middle and a last substep
+                    if ((r = loadState(snap)) != CRB200_OK || (r = stepMany(std::min(trial, 3))) != CRB200_OK)
+                        break;
                     if ((r = loadState(snap)) != CRB200_OK)
                         break;
                     if ((r = cudaFail(cudaEventRecord(e0, stream), "autotune event")) != CRB200_OK)
