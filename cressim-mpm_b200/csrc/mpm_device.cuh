@@ -986,10 +986,11 @@ namespace crb200
         return R;
     }
 
-    // The same for a matrix whose singular values lie within a factor of 1.73 of each other and
-    // whose determinant is positive: R^T is then Newton's iteration X <- (X + X^-T) / 2 on the scaled
-    // matrix (Higham 1986), which converges quadratically to the polar factor.  The test is on the
-    // Frobenius distance of X^T X from the identity at mean square singular value 1; inside it
+    // The same for a matrix near a rotation, whose determinant is positive: R^T is then Newton's iteration
+    // X <- (X + X^-T) / 2 on the scaled matrix (Higham 1986), which converges quadratically to the polar
+    // factor.  The test is on the Frobenius distance of X^T X from the identity at mean square singular
+    // value 1, at most 1/2: singular values within a factor of 1.46 of each other at most, of 1.44 where the
+    // middle one lies halfway.  Inside it
     // pbNeedsFp64 never holds, so no case of the double-precision redo comes here.  The last step
     // changed X by less than 1.8e-4, which leaves its square, below rounding.
     //
