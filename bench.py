@@ -246,7 +246,7 @@ def run_sdf(args, rank, world, local):
     e2e_ms = max_over_ranks(e0.elapsed_time(e1), world)
     leaves = -(-len(T) // 8)
     p2 = 1 << max(0, (leaves - 1).bit_length())
-    h2d = 16 * (3 * 8 * p2 + 4 * 2 * p2)  # triangle records + tree nodes the library uploads
+    h2d = 16 * (4 * 8 * p2 + 7 * 2 * p2)  # triangle records + tree nodes the library uploads
     peak, peak_kind = hbm_peak()
     grad_bytes = 20.0 * n  # read one distance, write one float4 per node (neighbours from cache)
     grad_gbs = grad_bytes * args.steps / (k_grad / 1e3) / 1e9

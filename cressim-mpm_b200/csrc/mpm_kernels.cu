@@ -1,24 +1,26 @@
 // sm_100a kernels of the B200 MPM substep engine and the host Solver that launches them.
 //
 // One substep (MLS-MPM; the reference's GpuMlsMpmSolver::step, gpu_mls_mpm_solver.cu:102-109):
-//   1. gatherShapes   scene shapes -> compact table (shapes may change between substeps); a launch
-//                     of its own only where the previous grid update could not do it
+//   1. gatherShapes   scene shapes -> compact table (shapes may change between substeps), by the
+//                     first CTAs of sortBlocks; a launch of its own beside the block-ordered sort
 //   2. bin            per particle: cell key (block-major), rank among its cell's particles, cell
 //                     and block counts (warp-aggregated atomics), and the list of active blocks;
 //                     done by the previous G2P when it can be
-//   3. sortBlocks     over the listed blocks only: the start of every cell, the work items of the
-//                     accumulation and the list of touched blocks
+//   3. sortBlocks     over the listed blocks only: the start of every cell, the end of the block
+//                     and the list of touched blocks
 //   4. place          particle ids into their cells' slots (cells contiguous in key order; arrival
 //                     order inside a cell; the canonical order is produced on request), and the
 //                     P2G records and cut masks that the previous G2P did not leave
-//   5. accumulate     one CTA per work item: particles -> shared-memory 6x6x6 node tile -> one
-//                     float4 vector atomic per touched node into the accumulation grid
+//   5. accumulate     64 threads or more per active block: particles -> shared-memory 6x6x6 node
+//                     tile -> one float4 vector atomic per touched node into the accumulation grid
 //   6. gridUpdate     touched blocks only: momentum -> velocity, SDF contact/friction, domain BC,
 //                     and the accumulation grid is zeroed as it is consumed
 //   7. g2p            particle order: 27-node gather, APIC matrix, advection, push-out, F update,
 //                     and the next substep's record and binning
-// The launches are a dependent chain (chainStart).  Deterministic substeps and the cell-ordered
-// path sort by block in an order that does not depend on arrival: bin, scan (3 kernels), scatter.
+// The launches are a dependent chain (chainStart).  Deterministic substeps order the ids of each
+// cell after placing (cellOrder) and sum block tiles; the order of the lists does not matter to
+// them.  The cell-ordered path, PB-MPM without iterations and the canonical permutation sort by
+// block in an order that does not depend on arrival: bin, scan (3 kernels), cellStarts, scatter.
 // PB-MPM runs 6-8 `iterations` times per step plus an integration kernel (gpu_pb_mpm_solver.cu:
 // 102-113); standard MPM carries a node force tile (gpu_standard_mpm_solver.cu:177-184).
 
@@ -355,7 +357,9 @@ namespace crb200
     //    one over the active ones, and the shape gather beside them).  It is bound by latency: one
     //    dependent chain per warp, so the counters are advanced once per CTA.  Binning to placing on
     //    the 1.6M-particle slab: 58 -> 34 us a substep; 64 scenes, 1.3M particles: 76 -> 36 us; 4096
-    //    particles: 37 -> 14 us, with 5 launches a substep instead of 12.
+    //    particles: 37 -> 14 us, with 5 launches a substep instead of 12.  At 6 CTAs per SM the shape
+    //    gather spills; 4 CTAs, which it does not, make no difference (4096 particles, 64k, the slab
+    //    and 64 scenes all within 1 %).
     __global__ void __launch_bounds__(256, 6) k_sortBlocks(const __grid_constant__ StepParams p, SceneTable sc, int shapeCtas,
                                                         const int *__restrict__ shapeIds, CrB200ShapeData shd,
                                                         CrB200GeometryData ge, ShapeRec *__restrict__ shapeTable,
@@ -683,11 +687,8 @@ namespace crb200
             sortedIds[slot] = i;
     }
 
-    // Absolute start of every cell of the active blocks (one warp per block, lane l scanning cells l
-    // and l + 32): the block's start plus the exclusive prefix of its cell counts, which are cleared
-    // for the next binning.
-    // Deterministic substeps: each cell's slots hold its particle ids in ascending order (the
-    // scatter places them in arrival order).  One 64-thread CTA per active block: the block's ids
+    // Deterministic substeps: each cell's slots hold its particle ids in ascending order (k_place
+    // leaves them in arrival order).  One 64-thread CTA per active block: the block's ids
     // go to shared memory (coalesced), thread c insertion-sorts cell c's segment, and they go back;
     // a block larger than the buffer sorts in place in global memory.
     constexpr unsigned kCellOrderCap = 2048;
@@ -733,6 +734,9 @@ namespace crb200
         }
     }
 
+    // Block-ordered sort: absolute start of every cell of the active blocks (one warp per block, lane l
+    // scanning cells l and l + 32): the block's start plus the exclusive prefix of its cell counts, which
+    // are cleared for the next binning.
     __global__ void __launch_bounds__(256) k_cellStarts(const SortHeader *__restrict__ hdr,
                                                         const unsigned *__restrict__ activeList,
                                                         const unsigned *__restrict__ blockStart,
@@ -1684,7 +1688,7 @@ namespace crb200
                 }
     }
 
-    // Cut masks of the current positions (bit a*9 + b*3 + c), for inspection.
+    // Cut masks of the current positions (bit a*9 + b*3 + c): PB-MPM's, for all iterations of a step.
     //    Multi: every particle gets a mask (zero in scenes without a slicer).
     template <bool Multi>
     __global__ void k_cutMasks(const __grid_constant__ StepParams p0, SceneTable sc, const float4 *__restrict__ xm,
@@ -1866,9 +1870,12 @@ namespace crb200
     // 440 us, 10 PB-MPM steps at 9k 2235 -> 2170 us, no difference at 1.6M.
     //
     // Single scenes of up to kEarlyParticles also let the next kernel's CTAs in while the last of
-    // theirs run: 4096 particles 291 -> 275 us, 13.8k 301 -> 287 us, PB-MPM at 16k 435 -> 422 us.
-    // Above, the CTAs that come early crowd on the SMs that happen to be free, and their kernel ends
-    // later: standard MPM at 33k 427 -> 551 us, PB-MPM at 37k 443 -> 465 us, batches alike.
+    // theirs run: 10 substeps of 10.6k particles 241 -> 229 us, standard MPM 310 -> 289, PB-MPM steps of
+    // 5 iterations at 22k 904 -> 845.  Above, the CTAs that come early crowd on the SMs that happen to be
+    // free, and their kernel ends later: standard MPM at 33k 427 -> 551 us, PB-MPM at 37k 443 -> 465 us,
+    // batches alike.  Several solvers on streams of their own pay for it (4 of 4096 particles 320 -> 342 us
+    // for 10 substeps of all, 16 of them 957 -> 1027), but are twice as fast as with the launches
+    // before the chain all the same (628 and 2360).
     constexpr unsigned kEarlyParticles = 24000;
     template <class... P>
     struct Chained
@@ -2274,7 +2281,7 @@ namespace crb200
     {
         auto run = [&](auto split, unsigned ctas) {
             constexpr int S = decltype(split)::value;
-            chained(k_accumulate<Mode, Multi, Det, S>, ctas, 64 * kGroups<Mode, S>, 0, stream)(
+            chained(k_accumulate<Mode, Multi, Det, S>, ctas, 64 * kGroups<S>, 0, stream)(
                 p, sc, hdr, active, ends, ids, starts, records, cutMasks, grid, gridF, Det ? detTiles : nullptr,
                 Det ? detTilesF : nullptr);
         };

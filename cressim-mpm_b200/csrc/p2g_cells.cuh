@@ -414,14 +414,14 @@ namespace crb200
     }
 
     // Groups of 64 threads in a CTA of the cell accumulation (see k_accumulate).
-    template <int Mode, int Split>
+    template <int Split>
     constexpr int kGroups = Split == 4 ? 6 : Split;
 
     // Shared memory of a CTA of the cell accumulation, whose groups may each have a block of their own.
-    template <int Mode, bool Multi, int Split>
+    template <bool Multi, int Split>
     struct AccumulateShared
     {
-        static constexpr int kWarps = 2 * kGroups<Mode, Split>;
+        static constexpr int kWarps = 2 * kGroups<Split>;
         // Node tile of each warp: momentum and mass of node (x, y, z) at x + kPitch (y + 6 z).  With a
         // pitch of 12 the 8 lanes of a 16-byte access (4 cells in x, 2 in y) cover all bank groups;
         // the widest CTAs, with 8 or 12 tiles, would pass 48 KB and take two-way conflicts.  One array of
@@ -429,16 +429,16 @@ namespace crb200
         // 1.6M particles 212 -> 209 us, of 85k 31.3 -> 31.1 us.
         static constexpr int kPitch = Split <= 2 ? 12 : kTileEdge, kTileSlots = kPitch * kTileEdge * kTileEdge;
         float4 tile[kWarps][kTileSlots];
-        unsigned start[kGroups<Mode, Split>][65];
-        unsigned ov[kGroups<Mode, Split>][65];
-        unsigned warpTot[kGroups<Mode, Split>];
-        StepParams p[Multi ? kGroups<Mode, Split> : 1]; // Multi: the current block's scene parameters
+        unsigned start[kGroups<Split>][65];
+        unsigned ov[kGroups<Split>][65];
+        unsigned warpTot[kGroups<Split>];
+        StepParams p[Multi ? kGroups<Split> : 1]; // Multi: the current block's scene parameters
     };
 
     // The active blocks of a CTA, each worked on by a team of Step groups: Split groups, all on one block at a
     // time, or single groups with blocks of their own.
     template <int Mode, bool Multi, bool Det, int Split, int Step>
-    __device__ __forceinline__ void accumulateBlocks(AccumulateShared<Mode, Multi, Split> &sh, const StepParams &p0,
+    __device__ __forceinline__ void accumulateBlocks(AccumulateShared<Multi, Split> &sh, const StepParams &p0,
                                                      const SceneTable &sc, unsigned nAct,
                                                      const unsigned *__restrict__ activeList,
                                                      const unsigned *__restrict__ blockEnd,
@@ -452,7 +452,7 @@ namespace crb200
         constexpr bool kWhole = Step == Split; // one team; groups past it have nothing to do
         constexpr int kThreads = 64 * Step, kWarps = 2 * Step;
         constexpr unsigned kRun = (unsigned)(kCellRun * Step); // particles of a cell its threads take
-        constexpr int kPitch = AccumulateShared<Mode, Multi, Split>::kPitch, kTileSlots = AccumulateShared<Mode, Multi, Split>::kTileSlots;
+        constexpr int kPitch = AccumulateShared<Multi, Split>::kPitch, kTileSlots = AccumulateShared<Multi, Split>::kTileSlots;
         if (kWhole && threadIdx.x >= (unsigned)kThreads)
             return;
         const unsigned team = kWhole ? 0u : threadIdx.x >> 6;
@@ -474,7 +474,7 @@ namespace crb200
         constexpr bool kAhead = !(Mode == 2 && Split > 1);
         const int passes = Mode == 2 ? 2 : 1;
         const int cx = cell & 3, cy = (cell >> 2) & 3, cz = cell >> 4;
-        for (unsigned ab = blockIdx.x + team * gridDim.x; ab < nAct; ab += gridDim.x * (kWhole ? 1u : (unsigned)kGroups<Mode, Split>))
+        for (unsigned ab = blockIdx.x + team * gridDim.x; ab < nAct; ab += gridDim.x * (kWhole ? 1u : (unsigned)kGroups<Split>))
         {
             const unsigned b = activeList[ab];
             const unsigned si = Multi ? (unsigned)sceneOfBlock(sc, b) : 0u;
@@ -693,7 +693,7 @@ namespace crb200
     //     88k in 511 blocks 345 -> 334, PB-MPM 1344 -> 1332, standard 516 -> 518 (and 93k in 996, a last
     //     round of few blocks, 390 -> 368, 1558 -> 1484 and 586 -> 603).
     template <int Mode, bool Multi, bool Det, int Split>
-    __global__ void __launch_bounds__(64 * kGroups<Mode, Split>, Split == 1 ? (Multi ? 5 : 6) : (Split == 2 ? 3 : 1)) k_accumulate(const __grid_constant__ StepParams p0, SceneTable sc, const SortHeader *__restrict__ hdr,
+    __global__ void __launch_bounds__(64 * kGroups<Split>, Split == 1 ? (Multi ? 5 : 6) : (Split == 2 ? 3 : 1)) k_accumulate(const __grid_constant__ StepParams p0, SceneTable sc, const SortHeader *__restrict__ hdr,
                                                        const unsigned *__restrict__ activeList,
                                                        const unsigned *__restrict__ blockEnd,
                                                        const unsigned *__restrict__ sortedIds,
@@ -704,7 +704,7 @@ namespace crb200
                                                        float4 *__restrict__ tilesF)
     {
         chainStart(p0.earlyNext);
-        __shared__ AccumulateShared<Mode, Multi, Split> sh;
+        __shared__ AccumulateShared<Multi, Split> sh;
         const unsigned nAct = hdr->numActiveBlocks;
         // each warp clears its own tile while the number of blocks is on its way
         for (int t = threadIdx.x & 31; t < sh.kTileSlots; t += 32)

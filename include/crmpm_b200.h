@@ -306,8 +306,9 @@ CRB200_API int CrB200SolverSetOption(CrB200SolverHandle solver, int option, int 
 
 /* Phase timing (CRB200_OPT_PHASE_TIMING on): CUDA-event milliseconds accumulated per phase on the
  * solver stream since the last reset, and the number of substeps they cover.  Phases:
- * 0 shape gather + binning + scan + scatter + cut masks + per-block cell sort, 1 P2G (particle
- * records + cell accumulation), 2 grid update, 3 G2P (PB-MPM: G2P plus the integration kernel).
+ * 0 shape gather + binning + block sort + placing (with the P2G records and cut masks that the
+ * previous G2P did not leave), 1 P2G (cell accumulation), 2 grid update, 3 G2P (which in MLS-MPM
+ * bins and writes the records of the next substep; PB-MPM: G2P plus the integration kernel).
  * On the resident path (CRB200_OPT_RESIDENT): 0 the call's start (shape gather, re-sort when due),
  * 1 the call's first P2G and the fused G2P -> P2G kernels, 2 grid updates, 3 the call's last G2P.
  * Synchronizes the solver stream. */
@@ -323,8 +324,8 @@ CRB200_API int CrB200SolverGetResidentKernelTime(CrB200SolverHandle solver, floa
 
 /* Launch-shape autotuner (no counterpart in the reference): times the candidate CTA counts of
  * the grid update (4, 8 or 16 per SM), the cell accumulation (1x or 2x its occupancy) and the
- * per-cell start computation (4 or 8 per SM) over substepsPerTrial substeps each (0: 8) from the current state, keeps the
- * fastest and restores the state; coupling forces of the trials are not reported.  Writes the
+ * block sort (6 or 12 per SM) over substepsPerTrial substeps each (0: 8) from the current state, keeps
+ * the fastest and restores the state; coupling forces of the trials are not reported.  Writes the
  * choice (update CTAs per SM, accumulation multiple, sort multiple) to outChoiceHost[3] if
  * given.  On the resident path (CRB200_OPT_RESIDENT) the second entry is the fused kernel's
  * multiple of its occupancy (1x or 2x) and the third is 1.  Needs a non-default solver stream;
